@@ -42,6 +42,26 @@ namespace {
 
 void default_tuning(gq_scene *s);
 
+// Bounding cylinders of the triangles and of the pair records' runs (layout.h), computed
+// on the device from the uploaded records; the caller has selected the scene's device.
+gq_status add_cylinders(gq_scene *s) {
+    if (s->dim != 3 || s->np < 1) return GQ_OK;
+    gqd::DevScene &d = s->dev;
+    const size_t bytes = 2 * sizeof(gq_cyl_t) * (size_t)s->np;
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess) return fail(GQ_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    s->allocs.push_back(p);
+    s->device_bytes += (int64_t)bytes;
+    gq_cyl_t *tri = (gq_cyl_t *)p, *run = tri + s->np;
+    e = gqd::build_cylinders(d, (int64_t)(s->image_bytes[0] / sizeof(gq_pair3_t)), tri, run);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    if (e != cudaSuccess) return fail_cuda(e, "bounding cylinders");
+    d.tri_cyl = tri;
+    d.run_cyl = run;
+    return GQ_OK;
+}
+
 // Linear BVH on the device (device/gpu_build.cu) straight into the traversal records.
 template <int D>
 gq_status build_on_device(gq_scene *s, const gq_build_opts &o) {
@@ -169,7 +189,7 @@ gq_status build_on_device(gq_scene *s, const gq_build_opts &o) {
     s->image_bytes[0] = s->np > 1 ? pair_bytes : 0;
     s->image_bytes[1] = prim_bytes;
     default_tuning(s);
-    return GQ_OK;
+    return add_cylinders(s);
 }
 
 template <int D>
@@ -290,6 +310,7 @@ gq_status build_scene(const float *vertices, int64_t nv, const int32_t *prims, i
     d.root_ref = img.root_ref;
     d.wroot_ref = img.wroot_ref;
     d.sroot_ref = img.sroot_ref;
+    if ((st = add_cylinders(s.get())) != GQ_OK) return st;
     *out = s.release();
     return GQ_OK;
 }
@@ -1159,6 +1180,7 @@ gq_status gq_scene_load(const char *path, int32_t device, gq_scene **out) {
     d.root_ref = h.root_ref;
     d.wroot_ref = h.wroot_ref;
     d.sroot_ref = h.sroot_ref;
+    if ((st = add_cylinders(s.get())) != GQ_OK) return st;
     *out = s.release();
     return GQ_OK;
 }

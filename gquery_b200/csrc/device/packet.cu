@@ -15,8 +15,10 @@ __device__ __forceinline__ float qget(const gq_vecs &v, int64_t i, int k) {
     return v.ptr[(int64_t)k * v.comp_stride + i * v.elem_stride];
 }
 
-template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT = false>
-__global__ void __launch_bounds__(kMaxBlock) k_cp_packet(DevScene s, gq_vecs q, int64_t n, const int32_t *perm,
+// Registers: 56 keep 36 warps on an SM (8,388,608 points: 48 / 56 / 64 registers 20.4-21.6 /
+// 19.4-20.2 / 22.4 ms); the sparse form needs 64 for its loops and is bound by latency.
+template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT, bool SPARSE>
+__global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q, int64_t n, const int32_t *perm,
                                                          gq_cp_out o, unsigned long long *counter) {
     const unsigned lane = threadIdx.x & 31u;
     // (ref, this lane's key) per entry; refs are the same in every lane
@@ -29,6 +31,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_cp_packet(DevScene s, gq_vecs q, 
         else
             return pkt::PStack<false>(plain);
     }();
+    extern __shared__ pkt::LeafBuf leaf_buf[];
+    pkt::LeafBuf *buf = SPARSE ? leaf_buf + (threadIdx.x >> 5) : nullptr;
     for (;;) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(counter, 32ull);
@@ -43,8 +47,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_cp_packet(DevScene s, gq_vecs q, 
         float r = kInf;
         int idx = -1;
         bool ovf = false;
-        pkt::closest_point<D, LAYOUT, MINFIRST, STK, COMPACT>(s, __ballot_sync(0xffffffffu, alive), p, r, idx, ovf,
-                                                                     stk);
+        pkt::closest_point<D, LAYOUT, MINFIRST, STK, COMPACT, SPARSE>(s, __ballot_sync(0xffffffffu, alive), p, r, idx, ovf,
+                                                             stk, buf);
         if (ovf && lane == 0 && s.err) atomicOr(s.err, GQ_DEVERR_STACK);
         if (alive) {
             if (D == 3)
@@ -55,28 +59,37 @@ __global__ void __launch_bounds__(kMaxBlock) k_cp_packet(DevScene s, gq_vecs q, 
     }
 }
 
-template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT = false>
+template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT = false, bool SPARSE = false>
 cudaError_t launch(const DevScene &s, int block, gq_vecs q, int64_t n, const int32_t *perm, const gq_cp_out &o,
                    unsigned long long *counter, cudaStream_t st) {
     static int bps[3] = {0, 0, 0}, n_sm = 0;
     int slot = block_slot(block);
     if (slot < 0) slot = 1, block = 128;
+    const size_t smem = SPARSE ? (size_t)(block / 32) * sizeof(pkt::LeafBuf) : 0;
     if (!bps[slot]) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT>, block, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, SPARSE>, block, smem);
         bps[slot] = b < 1 ? 1 : b;
     }
     const int64_t warps = (n + 31) / 32;
     const int64_t want = std::min<int64_t>((int64_t)bps[slot] * n_sm, (warps * 32 + block - 1) / block);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT><<<dim3((unsigned)want), block, 0, st>>>(s, q, n, perm, o,
-                                                                                                counter);
+    k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, SPARSE><<<dim3((unsigned)want), block, smem, st>>>(s, q, n, perm, o,
+                                                                                                   counter);
     return cudaGetLastError();
 }
+
+// Calls of fewer queries run the sparse form of the walk (packet.cuh), whose time is the
+// latency of the heaviest tiles; from here on the GPU has about fifteen tiles per
+// resident warp and the form with more warps wins.  Sparse against dense form, uniform points
+// on 1,310,720 triangles: 262,144 5.8 / 7.2 ms, 1,048,576 8.6 / 8.9, 2,097,152 11.5 / 10.7, 8,388,608
+// 23.9 / 19.9; 1,000,003 points near 327,680 triangles 1.25 / 1.55 ms.  Both forms give the
+// same answers bit for bit.
+constexpr int64_t kSparseBelow = 1 << 21;
 
 template <int D, int LAYOUT, bool MINFIRST>
 cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const int32_t *perm,
@@ -85,11 +98,114 @@ cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, c
         if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32, true>(s, t.block, q, n, perm, o, counter, st);
         return launch<D, LAYOUT, MINFIRST, pkt::kPStack, true>(s, t.block, q, n, perm, o, counter, st);
     }
+    if constexpr (D == 3 && LAYOUT == 0) {
+        if (n < kSparseBelow)
+            return t.stack == 32
+                       ? launch<D, LAYOUT, MINFIRST, 32, false, true>(s, t.block, q, n, perm, o, counter, st)
+                       : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, true>(s, t.block, q, n, perm, o, counter, st);
+    }
     if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32>(s, t.block, q, n, perm, o, counter, st);
     return launch<D, LAYOUT, MINFIRST, pkt::kPStack>(s, t.block, q, n, perm, o, counter, st);
 }
 
+// Bounding cylinder of triangles [first, first + count) (gq_cyl_t), in double, rounded
+// outward.  The axis is the sum of the triangles' area normals.
+__device__ void cylinder_of(const gq_tri_t *prims, int64_t first, int count, gq_cyl_t &out) {
+    double n[3] = {0, 0, 0}, lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    bool ok = true;
+    for (int j = 0; j < count; ++j) {
+        const gq_tri_t &t = prims[first + j];
+        const double v[3][3] = {{t.ax, t.ay, t.az}, {t.bx, t.by, t.bz}, {t.cx, t.cy, t.cz}};
+        double e[3][3], l2[3];
+        for (int k = 0; k < 3; ++k) {
+            l2[k] = 0;
+            for (int c = 0; c < 3; ++c) {
+                e[k][c] = v[(k + 1) % 3][c] - v[k][c];
+                l2[k] += e[k][c] * e[k][c];
+                lo[c] = fmin(lo[c], v[k][c]);
+                hi[c] = fmax(hi[c], v[k][c]);
+            }
+        }
+        const double m[3] = {e[0][1] * e[1][2] - e[0][2] * e[1][1], e[0][2] * e[1][0] - e[0][0] * e[1][2],
+                             e[0][0] * e[1][1] - e[0][1] * e[1][0]};
+        const double area = sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+        // height over the longest edge at least 1/64 of that edge
+        ok = ok && area * 64.0 >= fmax(l2[0], fmax(l2[1], l2[2])) && area > 1e-36;
+        for (int c = 0; c < 3; ++c) n[c] += m[c];
+    }
+    const double nl = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    ok = ok && nl > 0.0 && nl < INFINITY;
+    const float a[3] = {(float)(n[0] / nl), (float)(n[1] / nl), (float)(n[2] / nl)};
+    double c0[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])};
+    double half = 0, radius = 0;
+    float cf[3] = {0.f, 0.f, 0.f};
+    for (int pass = 0; pass < 2; ++pass) {  // the second with the centre at mid height
+        for (int c = 0; c < 3; ++c) cf[c] = (float)c0[c];
+        double h0 = INFINITY, h1 = -INFINITY;
+        radius = 0;
+        for (int j = 0; j < count; ++j) {
+            const gq_tri_t &t = prims[first + j];
+            const double v[3][3] = {{t.ax, t.ay, t.az}, {t.bx, t.by, t.bz}, {t.cx, t.cy, t.cz}};
+            for (int k = 0; k < 3; ++k) {
+                const double e[3] = {v[k][0] - cf[0], v[k][1] - cf[1], v[k][2] - cf[2]};
+                const double h = e[0] * a[0] + e[1] * a[1] + e[2] * a[2];
+                double g2 = 0;
+                for (int c = 0; c < 3; ++c) {
+                    const double g = e[c] - h * a[c];
+                    g2 += g * g;
+                }
+                h0 = fmin(h0, h);
+                h1 = fmax(h1, h);
+                radius = fmax(radius, sqrt(g2));
+            }
+        }
+        for (int c = 0; c < 3; ++c) c0[c] = cf[c] + 0.5 * (h0 + h1) * a[c];
+        half = fmax(fabs(h0), fabs(h1));
+    }
+    // 2^-20 of the cylinder's own size covers the rounding of the axis
+    const double slack = (radius + half) * 9.5367431640625e-07;
+    out.cx = cf[0];
+    out.cy = cf[1];
+    out.cz = cf[2];
+    out.radius = ok ? __double2float_ru(radius + slack) : kInf;
+    out.nx = ok ? a[0] : 0.f;
+    out.ny = ok ? a[1] : 0.f;
+    out.nz = ok ? a[2] : 0.f;
+    out.half = ok ? __double2float_ru(half + slack) : kInf;
+}
+
+__global__ void __launch_bounds__(128) k_tri_cyl(const gq_tri_t *prims, int64_t n, gq_cyl_t *out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) cylinder_of(prims, i, 1, out[i]);
+}
+
+// The walk meets the largest runs only: the two runs of a pair that is itself inside a run
+// are left out (they may start at the same triangle as the run around them).
+__global__ void __launch_bounds__(128) k_run_cyl(const gq_pair3_t *pairs, int64_t n, int32_t root, const gq_tri_t *prims,
+                                                 int64_t n_prims, gq_cyl_t *out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= 2 * n) return;
+    const uint32_t l = (uint32_t)pairs[i >> 1].sub_l, r = (uint32_t)pairs[i >> 1].sub_r;
+    if (l && r && (l >> 24) + (r >> 24) <= GQ_COLLAPSE_MAX && (i >> 1) != root) return;
+    const uint32_t sub = (i & 1) ? r : l;
+    const int64_t first = sub & 0xffffffu, count = sub >> 24;
+    if (count < 1 || first + count > n_prims) return;
+    cylinder_of(prims, first, (int)count, out[first]);
+}
+
 }  // namespace
+
+cudaError_t build_cylinders(const DevScene &s, int64_t n_pairs, gq_cyl_t *tri_cyl, gq_cyl_t *run_cyl) {
+    const gq_tri_t *prims = static_cast<const gq_tri_t *>(s.prims);
+    if (s.n_prims > 0)
+        k_tri_cyl<<<dim3((unsigned)((s.n_prims + 127) / 128)), 128>>>(prims, s.n_prims, tri_cyl);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    if (n_pairs > 0)
+        k_run_cyl<<<dim3((unsigned)((2 * n_pairs + 127) / 128)), 128>>>(
+            static_cast<const gq_pair3_t *>(s.pairs), n_pairs, s.root_ref, prims, s.n_prims, run_cyl);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_cp_packet(const DevScene &s, int layout, const Tune &t, gq_vecs q, int64_t n,
                              const int32_t *perm, const gq_cp_out &o, unsigned long long *counter, cudaStream_t st) {

@@ -89,6 +89,13 @@ struct PStack<true> {
     }
 };
 
+// square root within an ulp or two (one instruction)
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // squared distances from p to the nearest / farthest point of a box
 template <int D>
 __device__ __forceinline__ void box_sq(const float *lo, const float *hi, const float *p, float &a2, float &b2) {
@@ -103,27 +110,188 @@ __device__ __forceinline__ void box_sq(const float *lo, const float *hi, const f
     }
 }
 
-// Leaf: every lane that needs it tests the leaf's items against its query.
-template <int D>
-__device__ __forceinline__ void leaf(const DevScene &s, int ref, bool act, const float *p, float &r, int &idx) {
+// Squared distance below which x may have a point of the cylinder's set (gq_cyl_t).
+__device__ __forceinline__ float cyl_bound(const float4 &c, const float4 &n, float px, float py, float pz) {
+    const float ex = px - c.x, ey = py - c.y, ez = pz - c.z;
+    const float h = __fmaf_rn(ez, n.z, __fmaf_rn(ey, n.y, ex * n.x));
+    const float gx = __fmaf_rn(-h, n.x, ex), gy = __fmaf_rn(-h, n.y, ey), gz = __fmaf_rn(-h, n.z, ez);
+    const float t = sqrt_approx(__fmaf_rn(gz, gz, __fmaf_rn(gy, gy, gx * gx)));
+    const float a = fmaxf(fabsf(h) - n.w, 0.f), b = fmaxf(t - c.w, 0.f);
+    return __fmaf_rn(a, a, b * b);
+}
+
+// The bound a cylinder has to exceed for its triangles to be left untested: (sqrt(r) + eps)^2
+// for the squared radius r.  eps (2^-19 of the coordinates' size) is ten times the rounding
+// of cyl_bound and of the closest point that the triangle test forms together, so a triangle
+// that is left out would have had a key of at least r.  (The triangle test's barycentric
+// coordinates lose digits with the square of the distance over the triangle's size; up to a
+// thousand sizes away the point they give stays within the margin, and far beyond that its
+// own key means little.)
+__device__ __forceinline__ float cyl_limit(float r, float eps) {
+    const float s = sqrt_approx(r) + eps;
+    return s * s;
+}
+
+// Squared distance from p to the closest point of triangle abc: the arithmetic of
+// tri_closest (prim.cuh), rounding for rounding, with its seven regions chosen by selects
+// around one division instead of branches, for lanes that hold unrelated triangles.  The
+// closest point is base + e v + ac w: (a, ab) for a, the edges ab and ac and the inside,
+// (b, cb) for b and the edge bc, c alone; terms of zero weight add exactly nothing.
+__device__ __forceinline__ float tri_key(float px, float py, float pz, float ax, float ay, float az, float bx, float by,
+                                         float bz, float cx, float cy, float cz) {
+    const float abx = bx - ax, aby = by - ay, abz = bz - az;
+    const float acx = cx - ax, acy = cy - ay, acz = cz - az;
+    const float apx = px - ax, apy = py - ay, apz = pz - az;
+    const float d1 = gq_dot3(abx, aby, abz, apx, apy, apz);
+    const float d2 = gq_dot3(acx, acy, acz, apx, apy, apz);
+    const float bpx = px - bx, bpy = py - by, bpz = pz - bz;
+    const float d3 = gq_dot3(abx, aby, abz, bpx, bpy, bpz);
+    const float d4 = gq_dot3(acx, acy, acz, bpx, bpy, bpz);
+    const float cpx = px - cx, cpy = py - cy, cpz = pz - cz;
+    const float d5 = gq_dot3(abx, aby, abz, cpx, cpy, cpz);
+    const float d6 = gq_dot3(acx, acy, acz, cpx, cpy, cpz);
+    const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
+    const float s43 = d4 - d3, s56 = d5 - d6;
+    const bool in_a = (d1 <= 0.f) & (d2 <= 0.f);
+    const bool in_b = !in_a & (d3 >= 0.f) & (d4 <= d3);
+    const bool in_c = !in_a & !in_b & (d6 >= 0.f) & (d5 <= d6);
+    const bool vertex = in_a | in_b | in_c;
+    const bool on_ab = !vertex & (vc <= 0.f) & (d1 >= 0.f) & (d3 <= 0.f);
+    const bool on_ac = !vertex & !on_ab & (vb <= 0.f) & (d2 >= 0.f) & (d6 <= 0.f);
+    const bool on_bc = !vertex & !on_ab & !on_ac & (va <= 0.f) & (s43 >= 0.f) & (s56 >= 0.f);
+    float num = 1.f, den = va + vb + vc;
+    if (on_bc) num = s43, den = s43 + s56;
+    if (on_ac) num = d2, den = d2 - d6;
+    if (on_ab) num = d1, den = d1 - d3;
+    if (vertex) den = 1.f;
+    const float x = gq_div(num, den);
+    float v = vb * x, w = vc * x;
+    if (on_ab | on_bc) v = x, w = 0.f;
+    if (on_ac) v = 0.f, w = x;
+    if (vertex) v = 0.f, w = 0.f;
+    const bool from_b = in_b | on_bc;
+    const float ox = from_b ? bx : in_c ? cx : ax, oy = from_b ? by : in_c ? cy : ay, oz = from_b ? bz : in_c ? cz : az;
+    const float ux = on_bc ? cx - bx : abx, uy = on_bc ? cy - by : aby, uz = on_bc ? cz - bz : abz;
+    const float ex = px - ((ox + ux * v) + acx * w), ey = py - ((oy + uy * v) + acy * w),
+                ez = pz - ((oz + uz * v) + acz * w);
+    return gq_dot3(ex, ey, ez, ex, ey, ez);
+}
+
+// Pairs of a triangle and a lane that a sparse walk tests without bounds: two rounds of the
+// warp (32 / 64 / 96: 250,007 points near a 327,680-triangle surface 786 / 743 / 724 us,
+// 8,388,608 uniform points on 1,310,720 triangles 22.4 / 22.7 / 23.9 ms).
+constexpr int kRunPairs = 64;
+// Shared memory of one warp for the (triangle of a run, lane) pairs of leaf().
+struct LeafBuf {
+    float key[kRunPairs];
+    uint8_t pair[kRunPairs];  // triangle << 5 | lane
+    uint32_t sink[32];
+};
+static_assert(GQ_COLLAPSE_MAX <= 8, "a pair of leaf() fits a byte");
+
+// A run of at most GQ_COLLAPSE_MAX triangles from `first`, for the lanes in cmask.
+//
+// A triangle test costs about 100 instructions and nearly none improves a lane: of 584 per
+// tile of 32 queries (8,388,608 uniform points on 1,310,720 triangles; counts of a model of
+// the walk) 32 do.
+//
+// SPARSE, few lanes (at most kRunPairs pairs of a triangle and a lane): the lanes that need a
+// run are few where queries are sparse (8 of 32 near a surface, 4 for 2,003 points).  The
+// pairs are listed in shared memory, every lane of the warp tests one, and each query's
+// lane then takes its keys in the triangles' order.
+//
+// Otherwise the run's cylinder and then each triangle's disc (about 20 instructions each)
+// are tested first, and a triangle is left out when no lane can improve: 72 of 126 runs, and
+// 472 of the 584 triangles in all.
+//
+// A test that is left out would have left every lane's radius and winner as they are
+// (cyl_limit), and the pairs are taken in the order of the plain loop, so the walk
+// and its answers are those of testing every triangle, ties included.
+// RUNCYL: the run is a pair record's (run_cyl holds its cylinder).
+template <bool RUNCYL, bool SPARSE>
+__device__ __forceinline__ void run3(const DevScene &s, int first, int count, unsigned cmask, const float *p, float eps,
+                                     float &r, int &idx, LeafBuf *buf) {
+    const unsigned lane = threadIdx.x & 31u;
+    const bool act = (cmask >> lane) & 1u;
+    const int lanes = __popc(cmask), total = lanes * count;
+    if (SPARSE && total <= kRunPairs) {
+        const int rank = __popc(cmask & ((1u << lane) - 1u));
+        if (act)
+            for (int t = 0; t < count; ++t) buf->pair[t * lanes + rank] = (uint8_t)(t << 5 | lane);
+        __syncwarp();
+        for (int k0 = 0; k0 < total; k0 += 32) {
+            const int k = k0 + (int)lane;
+            const unsigned e = k < total ? buf->pair[k] : 0u;
+            const float x = __shfl_sync(0xffffffffu, p[0], e & 31u), y = __shfl_sync(0xffffffffu, p[1], e & 31u),
+                        z = __shfl_sync(0xffffffffu, p[2], e & 31u);
+            if (k < total) {
+                const int64_t j = 3 * (int64_t)(first + (int)(e >> 5));
+                const float4 t0 = ldg4(s.prims, j), t1 = ldg4(s.prims, j + 1), t2 = ldg4(s.prims, j + 2);
+                buf->key[k] = tri_key(x, y, z, t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x);
+            }
+        }
+        __syncwarp();
+        if (act)
+            for (int t = 0; t < count; ++t) {
+                const float key = buf->key[t * lanes + rank];
+                if (key < r) {
+                    r = key;
+                    idx = first + t;
+                }
+            }
+        __syncwarp();  // the buffer is free again
+        return;
+    }
+    float lim = cyl_limit(r, eps);
+    if (RUNCYL) {
+        const float4 c = ldg4(s.run_cyl, 2 * (int64_t)first), n = ldg4(s.run_cyl, 2 * (int64_t)first + 1);
+        if (!__any_sync(0xffffffffu, act && !(cyl_bound(c, n, p[0], p[1], p[2]) > lim))) return;
+    }
+    for (int j = first; j < first + count; ++j) {
+        const float4 c = ldg4(s.tri_cyl, 2 * (int64_t)j), n = ldg4(s.tri_cyl, 2 * (int64_t)j + 1);
+        const bool need = act && !(cyl_bound(c, n, p[0], p[1], p[2]) > lim);
+        if (!__any_sync(0xffffffffu, need)) continue;
+        const float4 t0 = ldg4(s.prims, 3 * (int64_t)j), t1 = ldg4(s.prims, 3 * (int64_t)j + 1),
+                     t2 = ldg4(s.prims, 3 * (int64_t)j + 2);
+        if (need) {
+            float pt[3], u, v;
+            tri_closest<true>(p[0], p[1], p[2], t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x, pt, &u, &v);
+            const float ex = p[0] - pt[0], ey = p[1] - pt[1], ez = p[2] - pt[2];
+            const float key = gq_dot3(ex, ey, ez, ex, ey, ez);
+            if (key < r) {
+                r = key;
+                idx = j;
+                lim = cyl_limit(r, eps);
+            }
+        }
+    }
+}
+
+// Leaf: every lane that needs it (cmask) tests the leaf's items against its query.
+template <int D, bool RUNCYL, bool SPARSE>
+__device__ __forceinline__ void leaf(const DevScene &s, int ref, unsigned cmask, const float *p, float eps, float &r,
+                                     int &idx, LeafBuf *buf) {
+    const bool act = (cmask >> (threadIdx.x & 31u)) & 1u;
     // a run of a collapsed subtree (bit 30 clear): first in bits 0-23, count in 24-29;
     // an ordinary leaf ~first (first < 2^30, so bit 30 set) runs to its last item
     const bool run = (ref & 0x40000000) == 0;
     int j = run ? (ref & 0xffffff) : ~ref;
     const int end = run ? j + ((ref >> 24) & 0x3f) : 0;
     if (run && end == j) return;  // an empty run (INT32_MIN, an unused wide slot): nothing to test
+    if (D == 3 && run) {
+        run3<RUNCYL, SPARSE>(s, j, end - j, cmask, p, eps, r, idx, buf);
+        return;
+    }
     for (;;) {
         bool last;
         if (D == 3) {
+            // a leaf of more than GQ_COLLAPSE_MAX triangles, or a device-built tree's
+            const float4 c = ldg4(s.tri_cyl, 2 * (int64_t)j), n = ldg4(s.tri_cyl, 2 * (int64_t)j + 1);
             const float4 t0 = ldg4(s.prims, 3 * (int64_t)j), t1 = ldg4(s.prims, 3 * (int64_t)j + 1),
                          t2 = ldg4(s.prims, 3 * (int64_t)j + 2);
-            last = run ? j + 1 == end : (fbits(t2.z) & GQ_ITEM_LAST) != 0;
-            if (act) {
-                float pt[3], u, v;
-                tri_closest<true>(p[0], p[1], p[D - 1], t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x, pt, &u,
-                                  &v);
-                const float ex = p[0] - pt[0], ey = p[1] - pt[1], ez = p[D - 1] - pt[2];
-                const float key = gq_dot3(ex, ey, ez, ex, ey, ez);
+            last = (fbits(t2.z) & GQ_ITEM_LAST) != 0;
+            if (act && !(cyl_bound(c, n, p[0], p[1], p[D - 1]) > cyl_limit(r, eps))) {
+                const float key = tri_key(p[0], p[1], p[D - 1], t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x);
                 if (key < r) {
                     r = key;
                     idx = j;
@@ -155,12 +323,18 @@ __device__ __forceinline__ void leaf(const DevScene &s, int ref, bool act, const
 // 1: quantised 8-wide nodes (3D only).  STK: entries of the caller's stack `stk`; the
 // warp stops with `ovf` set rather than overflow it.
 // COMPACT: the stack of PStack<true> (FP16 keys, one node word per warp).
-template <int D, int LAYOUT, bool MINFIRST, int STK = kPStack, bool COMPACT = false>
+// SPARSE (3D, LAYOUT 0): for calls whose time is the latency of a few walks rather than
+// their number: run3's pairs, and the children brought into L1 ahead (+20% on 262,144
+// points, -5% on 8,388,608).  buf: this warp's LeafBuf in shared memory.
+template <int D, int LAYOUT, bool MINFIRST, int STK = kPStack, bool COMPACT = false, bool SPARSE = false>
 __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, const float *p, float &r, int &idx,
-                                              bool &ovf, PStack<COMPACT> stk) {
+                                              bool &ovf, PStack<COMPACT> stk, LeafBuf *buf = nullptr) {
     const unsigned lane = threadIdx.x & 31u;
     const bool mine = (mask >> lane) & 1u;
     if (!mine) r = 0.f;  // never needs a node
+    float eps = 0.f;
+    if (D == 3) eps = (fmaxf(fmaxf(fabsf(p[0]), fabsf(p[1])), fabsf(p[D - 1])) + s.coord_bound) * 1.9073486e-06f;  // 2^-19
+    const unsigned sink = SPARSE ? (unsigned)__cvta_generic_to_shared(&buf->sink[lane]) : 0u;
     int cur = LAYOUT ? s.wroot_ref : s.root_ref;
     unsigned cmask = mask;
     int sp = -1;
@@ -183,7 +357,7 @@ __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, 
         }
         const bool act = (cmask >> lane) & 1u;
         if (cur < 0) {
-            leaf<D>(s, cur, act, p, r, idx);
+            leaf<D, LAYOUT == 0, SPARSE>(s, cur, cmask, p, eps, r, idx, buf);
             cur = kNone;
             continue;
         }
@@ -206,6 +380,18 @@ __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, 
                 lo[1][0] = b.x; lo[1][D - 1] = b.y; hi[1][0] = b.z; hi[1][D - 1] = b.w;
                 rl = rf.z ? (int)(0x80000000u | (unsigned)rf.z) : rf.x;
                 rr = rf.w ? (int)(0x80000000u | (unsigned)rf.w) : rf.y;
+            }
+            if (SPARSE) {
+                // Bring what a visit of either child reads first into L1 while the boxes are
+                // tested: half a warp per child, 4 bytes a lane to a place nobody reads.  An
+                // asynchronous copy needs no destination register, which a load would have to
+                // wait for at the next node.
+                const int cref = lane < 16 ? rl : rr;
+                const unsigned w = lane & 15u;
+                const char *from = (const char *)s.pairs + ((int64_t)(cref >= 0 ? cref : cur) * 64 + 4 * w);
+                if (cref < 0 && (cref & 0x40000000) == 0)  // a run: its triangles, at most 288 B
+                    from = (const char *)s.prims + ((int64_t)(cref & 0xffffff) * 48 + min(16 * w, 48 * ((cref >> 24) & 0x3fu) - 4));
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sink), "l"(from));
             }
             float a2l = kInf, b2l = kInf, a2r = kInf, b2r = kInf;
             if (act) {

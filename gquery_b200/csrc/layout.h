@@ -56,6 +56,18 @@ typedef struct {
     float cx, cy, cz, r;
 } gq_tsph_t;
 
+// Bounding cylinder of a set of triangles: centre, unit axis (their mean normal), radius
+// about the axis and half height along it.  With e = x - centre, h = axis . e and t the
+// length of e - h axis, every point of the set is at least
+// sqrt(max(|h| - half, 0)^2 + max(t - radius, 0)^2) from x (up to the rounding of that
+// expression).  Infinite radius and half height bound nothing (a set with a triangle too
+// thin for its own distance test to be trusted to that rounding).  Computed on the device
+// from the records, not kept in scene files.                               32 B
+typedef struct {
+    float cx, cy, cz, radius;
+    float nx, ny, nz, half;
+} gq_cyl_t;
+
 // 2D silhouette vertex: (a.xy, b.xy) | (c.xy, prim_id, flags)            32 B
 typedef struct {
     float ax, ay, bx, by;
