@@ -7,7 +7,9 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <thread>
@@ -31,6 +33,42 @@ gq_status fail(gq_status s, const std::string &msg) {
 }
 gq_status fail_cuda(cudaError_t e, const char *what) {
     return fail(GQ_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+namespace {
+struct ScratchPool {
+    cudaMemPool_t pool = nullptr;
+    int scenes = 0;
+};
+std::mutex g_pool_mu;
+std::map<int, ScratchPool> g_pools;  // by device
+}  // namespace
+
+cudaMemPool_t scratch_pool_retain(int device) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    ScratchPool &e = g_pools[device];
+    if (e.scenes++ == 0) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        uint64_t keep = kScratchKept;
+        if (cudaMemPoolCreate(&e.pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            e.pool = nullptr;
+        } else {
+            cudaMemPoolSetAttribute(e.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+    }
+    return e.pool;
+}
+
+void scratch_pool_release(int device) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    auto it = g_pools.find(device);
+    if (it == g_pools.end() || --it->second.scenes > 0) return;
+    if (it->second.pool) cudaMemPoolDestroy(it->second.pool);  // pending frees finish first
+    g_pools.erase(it);
 }
 }  // namespace gqi
 
@@ -60,6 +98,15 @@ gq_status add_cylinders(gq_scene *s) {
     d.tri_cyl = tri;
     d.run_cyl = run;
     return GQ_OK;
+}
+
+// What every scene with a device copy gets once its records are there.
+gq_status finish_device_scene(gq_scene *s) {
+    if (!s->allocs.empty()) {  // freed with them
+        s->pool = gqi::scratch_pool_retain(s->device);
+        s->pooled = true;
+    }
+    return add_cylinders(s);
 }
 
 // Linear BVH on the device (device/gpu_build.cu) straight into the traversal records.
@@ -189,7 +236,7 @@ gq_status build_on_device(gq_scene *s, const gq_build_opts &o) {
     s->image_bytes[0] = s->np > 1 ? pair_bytes : 0;
     s->image_bytes[1] = prim_bytes;
     default_tuning(s);
-    return add_cylinders(s);
+    return finish_device_scene(s);
 }
 
 template <int D>
@@ -310,7 +357,7 @@ gq_status build_scene(const float *vertices, int64_t nv, const int32_t *prims, i
     d.root_ref = img.root_ref;
     d.wroot_ref = img.wroot_ref;
     d.sroot_ref = img.sroot_ref;
-    if ((st = add_cylinders(s.get())) != GQ_OK) return st;
+    if ((st = finish_device_scene(s.get())) != GQ_OK) return st;
     *out = s.release();
     return GQ_OK;
 }
@@ -418,6 +465,10 @@ struct Scratch {
     }
 };
 
+cudaError_t scratch_alloc(const gq_scene *s, void **p, size_t bytes, cudaStream_t st) {
+    return s->pool ? cudaMallocFromPoolAsync(p, bytes, s->pool, st) : cudaMallocAsync(p, bytes, st);
+}
+
 // Per-call scratch: [work counter, 256 B][permutation, n int32][Morton sort workspace].
 // The counter feeds the persistent wide kernels; the rest is used when sorting.
 
@@ -434,7 +485,7 @@ gq_status prepare_order(const gq_scene *s, gq_vecs keys_from, int64_t n, const g
         if ((size_t)opts->scratch_bytes < need) return fail(GQ_ERR_INVALID, "scratch buffer too small");
         scr.p = opts->scratch;
     } else {
-        cudaError_t e = cudaMallocAsync(&scr.p, need, st);
+        cudaError_t e = scratch_alloc(s, &scr.p, need, st);
         if (e != cudaSuccess) return fail(GQ_ERR_NOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
         scr.owned = true;
         scr.st = st;
@@ -679,7 +730,7 @@ static gq_status order_impl(const gq_scene *s, gq_vecs points, int64_t n, int32_
         if ((size_t)scratch_bytes < need) return fail(GQ_ERR_INVALID, "scratch buffer too small");
         scr.p = scratch;
     } else {
-        cudaError_t e = cudaMallocAsync(&scr.p, need, cs);
+        cudaError_t e = scratch_alloc(s, &scr.p, need, cs);
         if (e != cudaSuccess) return fail(GQ_ERR_NOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
         scr.owned = true;
         scr.st = cs;
@@ -1180,7 +1231,7 @@ gq_status gq_scene_load(const char *path, int32_t device, gq_scene **out) {
     d.root_ref = h.root_ref;
     d.wroot_ref = h.wroot_ref;
     d.sroot_ref = h.sroot_ref;
-    if ((st = add_cylinders(s.get())) != GQ_OK) return st;
+    if ((st = finish_device_scene(s.get())) != GQ_OK) return st;
     *out = s.release();
     return GQ_OK;
 }

@@ -33,6 +33,17 @@ struct DeviceGuard {
     }
 };
 
+// Stream-ordered memory of the query calls' scratch on one device.  The device's default pool
+// hands its memory back to the system at every synchronisation, and a call that follows
+// one maps it again: 16 points 675 us instead of 180 us, 8,388,608 rays 9 to 400 ms instead
+// of 6.5 ms.  This pool keeps up to kScratchKept bytes while any scene lives on the
+// device, and goes with the last of them.
+constexpr uint64_t kScratchKept = 256ull << 20;  // a call of about 12 M queries
+// Counts a scene in (returning the device's pool, created with its first scene; null where it
+// cannot be) and out (destroying it with the last).
+cudaMemPool_t scratch_pool_retain(int device);
+void scratch_pool_release(int device);
+
 }  // namespace gqi
 
 struct gq_scene {
@@ -52,6 +63,8 @@ struct gq_scene {
     std::vector<float> wide16_words;  // and of their 16-bit bounds records
     std::vector<float> spair_words, sil_words;  // host copies of the SNCH pairs and silhouette records (idem)
     std::vector<void *> allocs;
+    bool pooled = false;  // counted in by scratch_pool_retain
+    cudaMemPool_t pool = nullptr;
     int64_t device_bytes = 0;
     gqd::DevScene dev{};
     gq_tuning tune[3] = {};
@@ -75,6 +88,7 @@ struct gq_scene {
     ~gq_scene() {
         if (device < 0 || allocs.empty()) return;
         gqi::DeviceGuard g(device);
+        if (pooled) gqi::scratch_pool_release(device);
         for (void *p : allocs) cudaFree(p);
     }
 
