@@ -419,6 +419,7 @@ gqd::Tune to_tune(const gq_scene *s, int kind, int variant) {
     r.block = t.block > 0 ? t.block : 128;
     const int need = (variant == GQ_VARIANT_WIDE8 || variant == GQ_VARIANT_WIDE16) ? s->wide_stack : s->exact_stack;
     r.stack = (t.stack == 32 && need <= 32) ? 32 : 0;
+    r.uncapped = s->dev.stack_cap == (1 << 30);
     return r;
 }
 
@@ -472,11 +473,12 @@ cudaError_t scratch_alloc(const gq_scene *s, void **p, size_t bytes, cudaStream_
 // Per-call scratch: [work counter, 256 B][permutation, n int32][Morton sort workspace].
 // The counter feeds the persistent wide kernels; the rest is used when sorting.
 
+// any_order: the kernel runs the queries in the caller's order unless one is given.
 // ray_dirs (3D rays): the rays are keyed by origin and direction (gq_ray_order mode 2),
 // which keeps the rays of a warp pointing alike.
 gq_status prepare_order(const gq_scene *s, gq_vecs keys_from, int64_t n, const gq_query_opts *opts,
                         cudaStream_t st, Scratch &scr, const int32_t **perm, unsigned long long **counter,
-                        const gq_vecs *ray_dirs = nullptr) {
+                        const gq_vecs *ray_dirs = nullptr, bool any_order = false) {
     *perm = nullptr;
     *counter = nullptr;
     const bool sorting = opts && !opts->order && opts->sort && n >= 2;
@@ -496,6 +498,7 @@ gq_status prepare_order(const gq_scene *s, gq_vecs keys_from, int64_t n, const g
         return GQ_OK;
     }
     if (!sorting) return GQ_OK;
+    if (any_order) return GQ_OK;
     int32_t *pp = (int32_t *)((char *)scr.p + kCounterBytes);
     char *rest = (char *)pp + align256((size_t)n * 4);
     const bool ray_keys = ray_dirs && s->dim == 3;
@@ -803,8 +806,10 @@ gq_status gq_intersect(const gq_scene *s, gq_vecs origin, gq_vecs dir, const flo
     Scratch scr;
     const int32_t *perm = nullptr;
     unsigned long long *counter = nullptr;
-    if ((st = prepare_order(s, origin, n, opts, cs, scr, &perm, &counter, &dir)) != GQ_OK) return st;
-    cudaError_t e = gqd::launch_ray(s->dev, v, to_tune(s, GQ_KIND_INTERSECT, v), origin, dir, r_max, n, perm,
+    const gqd::Tune tune = to_tune(s, GQ_KIND_INTERSECT, v);
+    if ((st = prepare_order(s, origin, n, opts, cs, scr, &perm, &counter, &dir, gqd::ray_any_order(s->dim, v, tune, n))) != GQ_OK)
+        return st;
+    cudaError_t e = gqd::launch_ray(s->dev, v, tune, origin, dir, r_max, n, perm,
                                     *out, counter, cs);
     if (e != cudaSuccess) return fail_cuda(e, "intersect launch");
     return GQ_OK;

@@ -51,6 +51,7 @@ struct Tune {
     int persist = 1;  // persistent warps with lane refill (per-thread traversal)
     int budget = 32;  // node visits between refills
     int block = 128;  // threads per block: 64, 128 or 256
+    bool uncapped = false;  // no stack limit is set on the scene
     int stack = 0;    // warp-coherent closest point: 32 = short stack (trees that fit), 0 = full depth
 };
 
@@ -64,6 +65,11 @@ cudaError_t launch_cp(const DevScene &s, int variant, const Tune &t, gq_vecs q, 
 // Rays over the quantised 8-wide BVH, one ray per group of 8 lanes (ray_group.cu).
 cudaError_t launch_ray_group(const DevScene &s, gq_vecs x, gq_vecs v, const float *r_max, int64_t n,
                              const int32_t *perm, const gq_ray_out &o, unsigned long long *counter, cudaStream_t st);
+// Whether a call's rays are fastest in the caller's order (those of ray_walk.cu's walk).
+bool ray_any_order(int dim, int variant, const Tune &t, int64_t n);
+// Rays over the quantised 8-wide BVH, the default (ray_walk.cu); answers as the per-lane walk's.
+cudaError_t launch_ray_walk(const DevScene &s, gq_vecs x, gq_vecs v, const float *r_max, int64_t n, const int32_t *perm,
+                            const gq_ray_out &o, unsigned long long *counter, cudaStream_t st);
 cudaError_t launch_ray(const DevScene &s, int variant, const Tune &t, gq_vecs x, gq_vecs v, const float *r_max,
                        int64_t n, const int32_t *perm, const gq_ray_out &o, unsigned long long *counter,
                        cudaStream_t st);
