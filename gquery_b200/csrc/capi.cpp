@@ -759,7 +759,9 @@ gq_status gq_closest_point(const gq_scene *s, gq_vecs q, int64_t n, const gq_cp_
     Scratch scr;
     const int32_t *perm = nullptr;
     unsigned long long *counter = nullptr;
-    if ((st = prepare_order(s, q, n, opts, cs, scr, &perm, &counter)) != GQ_OK) return st;
+    // up to one tile of the coherent walk: its answers do not depend on the order within
+    const bool any_order = v == GQ_VARIANT_COHERENT && n <= 32;
+    if ((st = prepare_order(s, q, n, opts, cs, scr, &perm, &counter, nullptr, any_order)) != GQ_OK) return st;
     cudaError_t e = gqd::launch_cp(s->dev, v, to_tune(s, GQ_KIND_CLOSEST_POINT, v), q, n, perm, *out, counter, cs);
     if (e != cudaSuccess) return fail_cuda(e, "closest_point launch");
     return GQ_OK;

@@ -65,6 +65,8 @@ cudaError_t launch_cp(const DevScene &s, int variant, const Tune &t, gq_vecs q, 
 // Rays over the quantised 8-wide BVH, one ray per group of 8 lanes (ray_group.cu).
 cudaError_t launch_ray_group(const DevScene &s, gq_vecs x, gq_vecs v, const float *r_max, int64_t n,
                              const int32_t *perm, const gq_ray_out &o, unsigned long long *counter, cudaStream_t st);
+// One closest point per warp, the per-lane walk's answers (cp_few.cu); for few queries.
+cudaError_t launch_cp_few(const DevScene &s, gq_vecs q, int64_t n, const gq_cp_out &o, cudaStream_t st);
 // Whether a call's rays are fastest in the caller's order (those of ray_walk.cu's walk).
 bool ray_any_order(int dim, int variant, const Tune &t, int64_t n);
 // Rays over the quantised 8-wide BVH, the default (ray_walk.cu); answers as the per-lane walk's.

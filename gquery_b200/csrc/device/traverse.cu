@@ -160,6 +160,7 @@ cudaError_t launch_cp(const DevScene &s, int variant, const Tune &t, gq_vecs q, 
         if (variant == GQ_VARIANT_WIDE8 && t.packet && s.dim == 3)
             return launch_cp_packet(s, t.sorted ? 1 : 2, t, q, n, perm, o, counter, st);
     }
+    if (variant == GQ_VARIANT_COHERENT && n < 32 && t.uncapped) return launch_cp_few(s, q, n, o, st);
     if (s.dim == 3)
         return wide ? launch_kind<3, false, true>(s, t, q, q, nullptr, n, perm, o, none, counter, st, q16)
                     : launch_kind<3, false, false>(s, t, q, q, nullptr, n, perm, o, none, counter, st);
