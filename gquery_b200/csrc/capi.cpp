@@ -518,6 +518,7 @@ struct gq_batch {
     int flags = 0;
     std::vector<gq_scene *> scenes;
     int64_t max_queries = 0;
+    bool uncapped = true;  // no scene had a stack limit when the batch was made
     gqd::DevScene *dev_scenes = nullptr;
     void *scratch = nullptr;
     int32_t *err = nullptr;
@@ -1299,6 +1300,7 @@ gq_status gq_batch_create(gq_scene *const *scenes, int32_t n_scenes, int64_t max
             return fail(GQ_ERR_INVALID, "batch scenes must share dimension and device");
         }
         views[(size_t)i] = s->dev;
+        b->uncapped &= s->dev.stack_cap == (1 << 30);
         b->scenes.push_back(scenes[i]);
     }
     DeviceGuard g(b->device);
@@ -1360,7 +1362,7 @@ gq_status gq_batch_run(gq_batch *b, const gq_batch_queries *cp, const gq_cp_out 
     bool all_wide = true;
     for (const gq_scene *s : b->scenes) all_wide &= s->has_wide;
     cudaError_t e = gqd::batch_run(b->dev_scenes, (int)b->scenes.size(), b->dim, kinds, co, ro, so,
-                                   (b->flags & GQ_BATCH_RAY_EXACT) || !all_wide ? 0 : 1,
+                                   (b->flags & GQ_BATCH_RAY_EXACT) || !all_wide ? 0 : b->uncapped ? 2 : 1,
                                    gqd::cp_mode_of(b->flags), gqd::sil_mode_of(b->flags),
                                    1.f, 128, true,
                                    b->scratch, b->max_queries, b->err, (cudaStream_t)stream);

@@ -50,11 +50,11 @@ __global__ void __launch_bounds__(kBlockR, 6) k_ray_walk(DevScene s, gq_vecs a, 
             }
             continue;
         }
-        if ((unsigned)L.cur < (unsigned)rayw::kNone) rayw::node<D>(s, L, stk);
+        if ((unsigned)L.cur < (unsigned)rayw::kNone) rayw::node<D>(s.wnodes, L, stk);
         const unsigned at_leaf = __ballot_sync(0xffffffffu, L.cur < 0);
         if (at_leaf) {
             const unsigned at_node = __ballot_sync(0xffffffffu, (unsigned)L.cur < (unsigned)rayw::kNone);
-            if (at_node == 0 || __popc(at_leaf) >= leaves) rayw::leaves<D>(s, L, stk, leaf_buf[threadIdx.x >> 5]);
+            if (at_node == 0 || __popc(at_leaf) >= leaves) rayw::leaves<D, false>(s.prims, L, stk, leaf_buf[threadIdx.x >> 5]);
         }
     }
 }

@@ -126,14 +126,14 @@ __device__ __forceinline__ void order2(uint32_t &a, uint32_t &b) {
 // each plane's t is one fma of q.  The keys carry the child's slot in their last three
 // bits, so the sort moves one word per child.
 template <int D>
-__device__ __forceinline__ void node(const DevScene &s, Lane<D> &L, int2 *stk) {
+__device__ __forceinline__ void node(const void *wnodes, Lane<D> &L, int2 *stk) {
     constexpr int F4 = (D == 3) ? 6 : 5;  // 16-byte words per node
     const int64_t at = F4 * (int64_t)L.cur;
-    const float4 h = ldg4(s.wnodes, at);
-    const uint4 q0 = __ldg(reinterpret_cast<const uint4 *>(s.wnodes) + at + 3);
-    const uint4 q1 = __ldg(reinterpret_cast<const uint4 *>(s.wnodes) + at + 4);
+    const float4 h = ldg4(wnodes, at);
+    const uint4 q0 = __ldg(reinterpret_cast<const uint4 *>(wnodes) + at + 3);
+    const uint4 q1 = __ldg(reinterpret_cast<const uint4 *>(wnodes) + at + 4);
     uint4 q2 = make_uint4(0, 0, 0, 0);
-    if (D == 3) q2 = __ldg(reinterpret_cast<const uint4 *>(s.wnodes) + at + 5);
+    if (D == 3) q2 = __ldg(reinterpret_cast<const uint4 *>(wnodes) + at + 5);
     const uint32_t meta = (uint32_t)fbits(D == 3 ? h.w : h.z);
     const int nc = (int)(meta >> 24);
     float A[D], Bn[D], Bf[D];
@@ -193,7 +193,7 @@ __device__ __forceinline__ void node(const DevScene &s, Lane<D> &L, int2 *stk) {
 #pragma unroll
         for (int k = 1; k < 8; ++k) key[0] = min(key[0], key[k]);
     }
-    const int *refs = reinterpret_cast<const int *>(s.wnodes) + 4 * (at + 1);
+    const int *refs = reinterpret_cast<const int *>(wnodes) + 4 * (at + 1);
 #pragma unroll
     for (int k = 7; k >= 1; --k)
         if (k < cnt) stk[++L.sp] = make_int2(__ldg(refs + (key[k] & 7u)), (int)(key[k] & ~7u));
@@ -201,16 +201,16 @@ __device__ __forceinline__ void node(const DevScene &s, Lane<D> &L, int2 *stk) {
 }
 
 template <int D>
-__device__ __forceinline__ float item_ray(const DevScene &s, int j, const float *p, const float *v, bool &last) {
+__device__ __forceinline__ float item_ray(const void *prims, int j, const float *p, const float *v, bool &last) {
     if (D == 3) {
-        const float4 t0 = ldg4(s.prims, 3 * (int64_t)j), t1 = ldg4(s.prims, 3 * (int64_t)j + 1),
-                     t2 = ldg4(s.prims, 3 * (int64_t)j + 2);
+        const float4 t0 = ldg4(prims, 3 * (int64_t)j), t1 = ldg4(prims, 3 * (int64_t)j + 1),
+                     t2 = ldg4(prims, 3 * (int64_t)j + 2);
         last = (fbits(t2.z) & GQ_ITEM_LAST) != 0;
         return tri_ray(p[0], p[1], p[D - 1], v[0], v[1], v[D - 1], t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x,
                        kInf);
     }
-    const float4 a = ldg4(s.prims, 2 * (int64_t)j);
-    last = (__ldg(reinterpret_cast<const int4 *>(s.prims) + 2 * (int64_t)j + 1).y & GQ_ITEM_LAST) != 0;
+    const float4 a = ldg4(prims, 2 * (int64_t)j);
+    last = (__ldg(reinterpret_cast<const int4 *>(prims) + 2 * (int64_t)j + 1).y & GQ_ITEM_LAST) != 0;
     return seg_ray(p[0], p[D - 1], v[0], v[D - 1], a.x, a.y, a.z, a.w);
 }
 
@@ -237,8 +237,9 @@ struct LeafBuf {
 // one after another, which is what a call of few rays waits for; so the pairs (item, lane) of all
 // waiting lanes are listed in shared memory and every lane of the warp tests one.
 // Each ray's lane then takes its keys in the items' order.
-template <int D>
-__device__ __forceinline__ void leaves(const DevScene &s, Lane<D> &L, const int2 *stk, LeafBuf &buf) {
+// MANY: the rays may be of different scenes (each lane passes its scene's items).
+template <int D, bool MANY>
+__device__ __forceinline__ void leaves(const void *prims, Lane<D> &L, const int2 *stk, LeafBuf &buf) {
     const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
     const bool here = L.cur < 0;
     // a run child (bit 30 clear) holds its count, an ordinary leaf ends at its last item
@@ -263,8 +264,13 @@ __device__ __forceinline__ void leaves(const DevScene &s, Lane<D> &L, const int2
             p[c] = __shfl_sync(0xffffffffu, L.p[c], e & 31u);
             v[c] = __shfl_sync(0xffffffffu, L.v[c], e & 31u);
         }
+        const void *items = prims;
+        if (MANY) {
+            const unsigned long long at = (unsigned long long)prims;
+            items = (const void *)__shfl_sync(0xffffffffu, at, e & 31u);
+        }
         bool last;
-        if (k < total) buf.key[k] = item_ray<D>(s, j, p, v, last);
+        if (k < total) buf.key[k] = item_ray<D>(items, j, p, v, last);
     }
     __syncwarp();
     int base = 0;
@@ -278,7 +284,7 @@ __device__ __forceinline__ void leaves(const DevScene &s, Lane<D> &L, const int2
         if (!run)
             for (int j = first;; ++j) {
                 bool last;
-                take<D>(L, item_ray<D>(s, j, L.p, L.v, last), j);
+                take<D>(L, item_ray<D>(prims, j, L.p, L.v, last), j);
                 if (last) break;
             }
         pop<D>(L, stk);

@@ -553,8 +553,11 @@ struct gq_server {
         if (S.m[0]) step_outputs(ring[0][S.cls], S.off[0], &co, nullptr, nullptr);
         if (S.m[1]) step_outputs(ring[1][S.cls], S.off[1], nullptr, &ro, nullptr);
         if (S.m[2]) step_outputs(ring[2][S.cls], S.off[2], nullptr, nullptr, &so);
-        bool all_wide = true;
-        for (const gq_scene *sc : scenes) all_wide &= sc->has_wide;
+        bool all_wide = true, uncapped = true;
+        for (const gq_scene *sc : scenes) {
+            all_wide &= sc->has_wide;
+            uncapped &= sc->dev.stack_cap == (1 << 30);
+        }
         const float share = S.sil_only ? sil_share : S.cls == kLarge ? large_share : 1.f;
         // One-warp blocks: the silhouette steps' one-warp blocks end all the time, and a
         // block of this step fits in the room any one of them leaves (a 128-thread block
@@ -563,7 +566,7 @@ struct gq_server {
         // sort are launches of large blocks that would wait the same way, and a small
         // step's requests are contiguous runs of one scene each already.
         cudaError_t e = gqd::batch_run(dev_scenes, (int)scenes.size(), D, kinds, co, ro, so,
-                                       (flags & GQ_BATCH_RAY_EXACT) || !all_wide ? 0 : 1,
+                                       (flags & GQ_BATCH_RAY_EXACT) || !all_wide ? 0 : uncapped ? 2 : 1,
                                        gqd::cp_mode_of(flags), gqd::sil_mode_of(flags), share, 32,
                                        S.cls == kLarge || !large_queries, S.scratch, step_queries, S.err, S.st);
         return e == cudaSuccess ? GQ_OK : fail_cuda(e, "server step");
