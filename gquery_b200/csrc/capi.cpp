@@ -473,12 +473,15 @@ cudaError_t scratch_alloc(const gq_scene *s, void **p, size_t bytes, cudaStream_
 // Per-call scratch: [work counter, 256 B][permutation, n int32][Morton sort workspace].
 // The counter feeds the persistent wide kernels; the rest is used when sorting.
 
+// tiles: where given, receives the order in which the warp-coherent walk starts its tiles
+// (gqd::tile_order).
 // any_order: the kernel runs the queries in the caller's order unless one is given.
 // ray_dirs (3D rays): the rays are keyed by origin and direction (gq_ray_order mode 2),
 // which keeps the rays of a warp pointing alike.
 gq_status prepare_order(const gq_scene *s, gq_vecs keys_from, int64_t n, const gq_query_opts *opts,
                         cudaStream_t st, Scratch &scr, const int32_t **perm, unsigned long long **counter,
-                        const gq_vecs *ray_dirs = nullptr, bool any_order = false) {
+                        const gq_vecs *ray_dirs = nullptr, bool any_order = false,
+                        const int32_t **tiles = nullptr) {
     *perm = nullptr;
     *counter = nullptr;
     const bool sorting = opts && !opts->order && opts->sort && n >= 2;
@@ -506,6 +509,11 @@ gq_status prepare_order(const gq_scene *s, gq_vecs keys_from, int64_t n, const g
                                       ray_keys ? 2 : 0, ray_keys ? *ray_dirs : gq_vecs{});
     if (e != cudaSuccess) return fail_cuda(e, "morton_order");
     *perm = pp;
+    if (tiles) {  // in the sort's workspace, free again
+        e = gqd::tile_order(s->dev, keys_from, n, pp, (int32_t *)rest, (int32_t *)scr.p + 32, st);
+        if (e != cudaSuccess) return fail_cuda(e, "tile order");
+        *tiles = (const int32_t *)rest;
+    }
     return GQ_OK;
 }
 
@@ -762,8 +770,12 @@ gq_status gq_closest_point(const gq_scene *s, gq_vecs q, int64_t n, const gq_cp_
     unsigned long long *counter = nullptr;
     // up to one tile of the coherent walk: its answers do not depend on the order within
     const bool any_order = v == GQ_VARIANT_COHERENT && n <= 32;
-    if ((st = prepare_order(s, q, n, opts, cs, scr, &perm, &counter, nullptr, any_order)) != GQ_OK) return st;
-    cudaError_t e = gqd::launch_cp(s->dev, v, to_tune(s, GQ_KIND_CLOSEST_POINT, v), q, n, perm, *out, counter, cs);
+    gqd::Tune tune = to_tune(s, GQ_KIND_CLOSEST_POINT, v);
+    const bool middle_first = v == GQ_VARIANT_COHERENT && s->dim == 3;  // 19.0 -> 18.2 ms for 8,388,608 points
+    if ((st = prepare_order(s, q, n, opts, cs, scr, &perm, &counter, nullptr, any_order,
+                            middle_first && n >= (1 << 22) ? &tune.tiles : nullptr)) != GQ_OK)
+        return st;
+    cudaError_t e = gqd::launch_cp(s->dev, v, tune, q, n, perm, *out, counter, cs);
     if (e != cudaSuccess) return fail_cuda(e, "closest_point launch");
     return GQ_OK;
 }
@@ -840,8 +852,12 @@ gq_status gq_closest_silhouette(const gq_scene *s, gq_vecs x, const float *r_max
     const int32_t *perm = nullptr;
     unsigned long long *counter = nullptr;
     gq_status st;
-    if ((st = prepare_order(s, x, n, opts, cs, scr, &perm, &counter)) != GQ_OK) return st;
-    cudaError_t e = gqd::launch_sil(s->dev, v, to_tune(s, GQ_KIND_SILHOUETTE, v), x, r_max, n, perm, *out, counter,
+    gqd::Tune tune = to_tune(s, GQ_KIND_SILHOUETTE, v);
+    const bool middle_first = v == GQ_VARIANT_COHERENT && s->dim == 3;
+    if ((st = prepare_order(s, x, n, opts, cs, scr, &perm, &counter, nullptr, false,
+                            middle_first && n >= (1 << 18) ? &tune.tiles : nullptr)) != GQ_OK)
+        return st;
+    cudaError_t e = gqd::launch_sil(s->dev, v, tune, x, r_max, n, perm, *out, counter,
                                     cs);
     if (e != cudaSuccess) return fail_cuda(e, "closest_silhouette launch");
     return GQ_OK;

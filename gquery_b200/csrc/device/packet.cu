@@ -18,7 +18,7 @@ __device__ __forceinline__ float qget(const gq_vecs &v, int64_t i, int k) {
 // Registers: 56 keep 36 warps on an SM (8,388,608 points: 48 / 56 / 64 registers 20.4-21.6 /
 // 19.4-20.2 / 22.4 ms); the sparse form needs 64 for its loops and is bound by latency.
 template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT, bool SPARSE>
-__global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q, int64_t n, const int32_t *perm,
+__global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q, int64_t n, const int32_t *perm, const int32_t *tiles,
                                                          gq_cp_out o, unsigned long long *counter) {
     const unsigned lane = threadIdx.x & 31u;
     // (ref, this lane's key) per entry; refs are the same in every lane
@@ -38,7 +38,7 @@ __global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q,
         if (lane == 0) base = atomicAdd(counter, 32ull);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= (unsigned long long)n) break;
-        const int64_t i = (int64_t)base + lane;
+        const int64_t i = (tiles ? 32 * (int64_t)__ldg(tiles + base / 32) : (int64_t)base) + lane;
         const bool alive = i < n;
         const int64_t qi = alive ? (perm ? (int64_t)__ldg(perm + i) : i) : 0;
         float p[D];
@@ -60,10 +60,10 @@ __global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q,
 }
 
 template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT = false, bool SPARSE = false>
-cudaError_t launch(const DevScene &s, int block, gq_vecs q, int64_t n, const int32_t *perm, const gq_cp_out &o,
+cudaError_t launch(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const int32_t *perm, const gq_cp_out &o,
                    unsigned long long *counter, cudaStream_t st) {
     static int bps[3] = {0, 0, 0}, n_sm = 0;
-    int slot = block_slot(block);
+    int block = t.block, slot = block_slot(block);
     if (slot < 0) slot = 1, block = 128;
     const size_t smem = SPARSE ? (size_t)(block / 32) * sizeof(pkt::LeafBuf) : 0;
     if (!bps[slot]) {
@@ -78,7 +78,7 @@ cudaError_t launch(const DevScene &s, int block, gq_vecs q, int64_t n, const int
     const int64_t want = std::min<int64_t>((int64_t)bps[slot] * n_sm, (warps * 32 + block - 1) / block);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, SPARSE><<<dim3((unsigned)want), block, smem, st>>>(s, q, n, perm, o,
+    k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, SPARSE><<<dim3((unsigned)want), block, smem, st>>>(s, q, n, perm, t.tiles, o,
                                                                                                    counter);
     return cudaGetLastError();
 }
@@ -95,17 +95,17 @@ template <int D, int LAYOUT, bool MINFIRST>
 cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const int32_t *perm,
                        const gq_cp_out &o, unsigned long long *counter, cudaStream_t st) {
     if (t.packet == 2) {  // the compact stack (FP16 keys, one node word per warp)
-        if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32, true>(s, t.block, q, n, perm, o, counter, st);
-        return launch<D, LAYOUT, MINFIRST, pkt::kPStack, true>(s, t.block, q, n, perm, o, counter, st);
+        if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32, true>(s, t, q, n, perm, o, counter, st);
+        return launch<D, LAYOUT, MINFIRST, pkt::kPStack, true>(s, t, q, n, perm, o, counter, st);
     }
     if constexpr (D == 3 && LAYOUT == 0) {
         if (n < kSparseBelow)
             return t.stack == 32
-                       ? launch<D, LAYOUT, MINFIRST, 32, false, true>(s, t.block, q, n, perm, o, counter, st)
-                       : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, true>(s, t.block, q, n, perm, o, counter, st);
+                       ? launch<D, LAYOUT, MINFIRST, 32, false, true>(s, t, q, n, perm, o, counter, st)
+                       : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, true>(s, t, q, n, perm, o, counter, st);
     }
-    if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32>(s, t.block, q, n, perm, o, counter, st);
-    return launch<D, LAYOUT, MINFIRST, pkt::kPStack>(s, t.block, q, n, perm, o, counter, st);
+    if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32>(s, t, q, n, perm, o, counter, st);
+    return launch<D, LAYOUT, MINFIRST, pkt::kPStack>(s, t, q, n, perm, o, counter, st);
 }
 
 // Bounding cylinder of triangles [first, first + count) (gq_cyl_t), in double, rounded

@@ -261,7 +261,7 @@ constexpr float kConeSlack = 1e-5f;
 
 template <int D>
 __device__ __forceinline__ bool cone_overlaps_fast(const float *lo, const float *hi, const float *axis, float half,
-                                                   float radius, const float *x, float dmin) {
+                                                   float radius, const float *x) {
     if (half >= GQ_PIO2_F) return true;  // |dA - pi/2| <= pi/2 <= h always holds
     float c[D], v[D], l2 = 0.f;
 #pragma unroll
@@ -313,7 +313,6 @@ __device__ __forceinline__ bool cone_overlaps_fast(const float *lo, const float 
     const float cos_sum = ch * cv - sh * sv;  // cos(h + h_v)
     if (cos_sum <= kConeSlack) return true;   // h + h_v >= pi/2
     const float sin_sum = sh * cv + ch * sv;  // sin(h + h_v), h + h_v in [0, pi/2)
-    (void)dmin;
     return dt <= sin_sum + kConeSlack;
 }
 

@@ -54,7 +54,8 @@ __device__ __forceinline__ void sil_write(const DevScene &s, const snch::Lane<D>
 // consecutive queries of the sorted order at a time.
 template <int D>
 __global__ void __launch_bounds__(kMaxBlock, 4) k_sil_packet(DevScene s, gq_vecs xq, const float *rmax_in, int64_t n,
-                                                       const int32_t *perm, gq_sil_out o, unsigned long long *counter) {
+                                                       const int32_t *perm, const int32_t *tiles, gq_sil_out o,
+                                                       unsigned long long *counter) {
     const unsigned lane = threadIdx.x & 31u;
     snch::Stack stk;
     for (;;) {
@@ -62,7 +63,7 @@ __global__ void __launch_bounds__(kMaxBlock, 4) k_sil_packet(DevScene s, gq_vecs
         if (lane == 0) base = atomicAdd(counter, 32ull);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= (unsigned long long)n) break;
-        const int64_t i = (int64_t)base + lane;
+        const int64_t i = (tiles ? 32 * (int64_t)__ldg(tiles + base / 32) : (int64_t)base) + lane;
         const bool alive = i < n;
         const int64_t qi = alive ? query_index(perm, i) : 0;
         snch::Lane<D> L;
@@ -651,6 +652,24 @@ __global__ void __launch_bounds__(256) k_read_probe(const uint4 *buf, int64_t n1
     if ((threadIdx.x & 31u) == 0) atomicXor(sink, acc);
 }
 
+// Tiles whose middle query lies in the middle half of the box (per axis) from the front of
+// the list, the others from its back, in any order.
+__global__ void __launch_bounds__(128) k_tile_order(DevScene s, gq_vecs q, int64_t n, const int32_t *perm, int32_t *tiles,
+                                                    int64_t n_tiles, int32_t *ends) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= n_tiles) return;
+    const int64_t qi = query_index(perm, min(32 * t + 16, n - 1));
+    bool mid = true;
+    for (int k = 0; k < s.dim; ++k) {
+        const float c = 0.5f * (s.root_lo[k] + s.root_hi[k]);
+        mid = mid && fabsf(qget(q, qi, k) - c) < 0.25f * (s.root_hi[k] - s.root_lo[k]);
+    }
+    if (mid)
+        tiles[atomicAdd(&ends[0], 1)] = (int32_t)t;
+    else
+        tiles[n_tiles - 1 - atomicAdd(&ends[1], 1)] = (int32_t)t;
+}
+
 inline dim3 grid_for(int64_t n) { return dim3((unsigned)((n + kBlock - 1) / kBlock)); }
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
@@ -662,6 +681,15 @@ size_t cub_temp_bytes(int64_t n) {
 }
 
 }  // namespace
+
+cudaError_t tile_order(const DevScene &s, gq_vecs q, int64_t n, const int32_t *perm, int32_t *tiles, int32_t *ends,
+                       cudaStream_t st) {
+    const int64_t n_tiles = (n + 31) / 32;
+    cudaError_t e = cudaMemsetAsync(ends, 0, 2 * sizeof(int32_t), st);
+    if (e != cudaSuccess) return e;
+    k_tile_order<<<grid_for(n_tiles), kBlock, 0, st>>>(s, q, n, perm, tiles, n_tiles, ends);
+    return cudaGetLastError();
+}
 
 size_t morton_scratch_bytes(int64_t n) {
     return 3 * align256((size_t)n * 4) + align256(cub_temp_bytes(n));
@@ -748,9 +776,9 @@ cudaError_t launch_sil(const DevScene &s, int variant, const Tune &t, gq_vecs x,
         const dim3 grid((unsigned)want);
         if (packet) {
             if (s.dim == 3)
-                k_sil_packet<3><<<grid, block, 0, st>>>(s, x, r_max, n, perm, o, counter);
+                k_sil_packet<3><<<grid, block, 0, st>>>(s, x, r_max, n, perm, t.tiles, o, counter);
             else
-                k_sil_packet<2><<<grid, block, 0, st>>>(s, x, r_max, n, perm, o, counter);
+                k_sil_packet<2><<<grid, block, 0, st>>>(s, x, r_max, n, perm, t.tiles, o, counter);
         } else {
             const int b = t.budget > 0 ? t.budget : 32;
             if (s.dim == 3)

@@ -44,6 +44,15 @@ size_t morton_scratch_bytes(int64_t n);
 cudaError_t morton_order(const DevScene &s, gq_vecs q, int64_t n, int32_t *perm, void *scratch, size_t scratch_bytes,
                          cudaStream_t st, int ray_mode = 0, gq_vecs ray_dir = gq_vecs{});
 
+// Writes the tiles 0 .. (n + 31) / 32 - 1 of the order `perm` to `tiles`, those in the middle of
+// the scene's box first: inside a closed mesh many parts of the surface are about equally
+// far, and a tile there takes up to ten times the average (silhouettes on 327,680 triangles: 15,215
+// steps within a quarter of the box, 1,150 on average), which the launch would wait for at
+// its end.  Silhouettes, 3D: 4,194,304 queries 29.8 -> 24.5 ms, 1,048,576 16.3 -> 14.3, 524,288 14.1 ->
+// 13.4; 2D polylines gain nothing.  `ends` is an 8-byte device word.
+cudaError_t tile_order(const DevScene &s, gq_vecs q, int64_t n, const int32_t *perm, int32_t *tiles, int32_t *ends,
+                       cudaStream_t st);
+
 // Launch choices for one query kind (picked by the autotuner or the defaults).
 struct Tune {
     int packet = 0;   // closest point: 1 = warp-coherent traversal
@@ -52,6 +61,7 @@ struct Tune {
     int budget = 32;  // node visits between refills
     int block = 128;  // threads per block: 64, 128 or 256
     bool uncapped = false;  // no stack limit is set on the scene
+    const int32_t *tiles = nullptr;  // warp-coherent walks: the order their tiles of 32 queries start in
     int stack = 0;    // warp-coherent closest point: 32 = short stack (trees that fit), 0 = full depth
 };
 

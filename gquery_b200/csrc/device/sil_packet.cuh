@@ -52,6 +52,7 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, unsigned m
             box_dist3(s.root_lo[0], s.root_lo[1], s.root_lo[2], s.root_hi[0], s.root_hi[1], s.root_hi[2], L.x[0],
                       L.x[1], L.x[D - 1], dmin_root, dmax_root);
     }
+    float lim2 = D == 2 ? snch::key_limit<D>(L.r) : 0.f;  // 2D: follows L.r
     unsigned cmask = __ballot_sync(0xffffffffu, mine && dmin_root <= L.r);
     int cur = cmask ? s.sroot_ref : kSilNone;
     int sp = -1;
@@ -62,7 +63,7 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, unsigned m
             while (sp >= 0) {
                 const int2 e = stk[sp--];
                 // pop-time test of the reference, per lane (snch.py:118)
-                const unsigned m = __ballot_sync(0xffffffffu, mine && __int_as_float(e.y) <= L.r);
+                const unsigned m = __ballot_sync(0xffffffffu, mine && __int_as_float(e.y) <= (D == 2 ? lim2 : L.r));
                 if (m) {
                     cur = e.x;
                     cmask = m;
@@ -75,12 +76,14 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, unsigned m
         const bool act = (cmask >> lane) & 1u;
         if (cur < 0) {
             if (cur != INT32_MIN) {  // INT32_MIN: leaf without silhouettes
+                const float before = L.r;
                 for (int j = ~cur;; ++j) {
                     const int flags = D == 2 ? fbits(ldg4(s.sils, 2 * (int64_t)j + 1).w)
                                              : fbits(ldg4(s.sils, 4 * (int64_t)j + 3).y);
                     if (act) snch::test_silhouette<D>(s, L, j);
                     if (flags & GQ_ITEM_LAST) break;
                 }
+                if (D == 2 && L.r != before) lim2 = snch::key_limit<D>(L.r);
             }
             cur = kSilNone;
             continue;
@@ -88,29 +91,23 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, unsigned m
         snch::PairView<D> P;
         snch::load_pair<D>(s, cur, P);
         bool hit[2] = {false, false};
-        float dm[2] = {kInf, kInf};
+        float dm[2] = {kInf, kInf};  // keys (snch::box_key)
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             if (act) {
-                float dmax;
-                if (D == 2)
-                    box_dist2(P.lo[c][0], P.lo[c][D - 1], P.hi[c][0], P.hi[c][D - 1], L.x[0], L.x[D - 1], dm[c],
-                              dmax);
-                else
-                    box_dist3(P.lo[c][0], P.lo[c][1], P.lo[c][D - 1], P.hi[c][0], P.hi[c][1], P.hi[c][D - 1], L.x[0],
-                              L.x[1], L.x[D - 1], dm[c], dmax);
-                hit[c] = dm[c] <= L.r;
+                dm[c] = snch::box_key<D>(P.lo[c], P.hi[c], L.x);
+                hit[c] = dm[c] <= (D == 2 ? lim2 : L.r);
                 // the node bound first: it rejects most of what the cone test rejects, for less
                 // (both must admit a child, so the order changes no decision)
                 if (hit[c]) hit[c] = !snch::child_free<D, kPacketCone>(s, P, c, L.x);
                 if ((P.half[c] >= 0.f) & hit[c])
-                    hit[c] = cone_overlaps_fast<D>(P.lo[c], P.hi[c], P.ax[c], P.half[c], P.rad[c], L.x, dm[c]);
+                    hit[c] = cone_overlaps_fast<D>(P.lo[c], P.hi[c], P.ax[c], P.half[c], P.rad[c], L.x);
             }
         }
         const unsigned m0 = __ballot_sync(0xffffffffu, hit[0]), m1 = __ballot_sync(0xffffffffu, hit[1]);
         if (m0 && m1) {
             const float k0 = warp_min(hit[0] ? dm[0] : kInf), k1 = warp_min(hit[1] ? dm[1] : kInf);
-            const bool second_first = k1 < k0;  // the nearer child (over the lanes) is entered first
+            const bool second_first = snch::key_less<D>(k1, k0);  // the nearer child (over the lanes) is entered first
             if (sp + 1 >= min(GQ_STACK_EXACT, s.stack_cap)) {
                 ovf = true;
                 break;

@@ -65,11 +65,12 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, const floa
                   x[D - 1], dmin_root, dmax_root);
     int sp = 0;  // entries on the stack (warp-uniform)
     if (dmin_root <= r_max) {
-        if (lane == 0) stk[0] = make_int2(s.sroot_ref, fbits(dmin_root));
+        if (lane == 0) stk[0] = make_int2(s.sroot_ref, fbits(0.f));  // admitted already
         sp = 1;
     }
     __syncwarp();
-    float R = r_max;  // warp's r_max
+    float R = r_max;  // warp's r_max, and in 2D the key of a box within it
+    float lim2 = D == 2 ? snch::key_limit<D>(r_max) : 0.f;
     bool ovf = false;
     while (sp > 0) {
         const int take = (sp + 32 <= kWarpStack - kReserve) ? min(sp, 32) : 1;
@@ -81,7 +82,7 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, const floa
         L.r = R;
         int2 push0 = make_int2(0, 0), push1 = make_int2(0, 0);  // the lane's entries, push1 on top
         int np = 0;
-        if (mine && __int_as_float(e.y) <= R) {
+        if (mine && __int_as_float(e.y) <= (D == 2 ? lim2 : R)) {
             if (e.x < 0) {
                 if (e.x != INT32_MIN)
                     for (int j = ~e.x;; ++j)
@@ -91,26 +92,20 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, const floa
                 snch::PairView<D> P;
                 snch::load_pair<D>(s, e.x, P);
                 bool hit[2];
-                float dm[2];
+                float dm[2];  // keys (snch::box_key)
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
-                    float dmax;
-                    if (D == 2)
-                        box_dist2(P.lo[c][0], P.lo[c][D - 1], P.hi[c][0], P.hi[c][D - 1], x[0], x[D - 1], dm[c],
-                                  dmax);
-                    else
-                        box_dist3(P.lo[c][0], P.lo[c][1], P.lo[c][D - 1], P.hi[c][0], P.hi[c][1], P.hi[c][D - 1],
-                                  x[0], x[1], x[D - 1], dm[c], dmax);
-                    hit[c] = dm[c] <= L.r;
+                    dm[c] = snch::box_key<D>(P.lo[c], P.hi[c], x);
+                    hit[c] = dm[c] <= (D == 2 ? lim2 : L.r);
                     // the node bound first: it rejects most of what the cone test rejects, for less
                     // (both must admit a child, so the order changes no decision)
                     if (hit[c]) hit[c] = !snch::child_free<D>(s, P, c, x);
                     if ((P.half[c] >= 0.f) & hit[c])
-                        hit[c] = cone_overlaps_fast<D>(P.lo[c], P.hi[c], P.ax[c], P.half[c], P.rad[c], x, dm[c]);
+                        hit[c] = cone_overlaps_fast<D>(P.lo[c], P.hi[c], P.ax[c], P.half[c], P.rad[c], x);
                 }
                 // push the farther first so the nearer is taken first (selects, not indexed
                 // arrays, so that nothing here lives in local memory)
-                const bool sw = dm[1] < dm[0];
+                const bool sw = snch::key_less<D>(dm[1], dm[0]);
                 const bool hf = sw ? hit[0] : hit[1], hn = sw ? hit[1] : hit[0];
                 const int2 ef = sw ? make_int2(P.refs[0], fbits(dm[0])) : make_int2(P.refs[1], fbits(dm[1]));
                 const int2 en = sw ? make_int2(P.refs[1], fbits(dm[1])) : make_int2(P.refs[0], fbits(dm[0]));
@@ -123,6 +118,7 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, const floa
         float m;
         int who;
         warp_argmin(L.r, m, who);
+        if (D == 2 && m != R) lim2 = snch::key_limit<D>(m);
         R = m;
         // push: lane 31's entries at the bottom, lane 0's on top
         const unsigned has1 = __ballot_sync(0xffffffffu, np >= 1), has2 = __ballot_sync(0xffffffffu, np >= 2);

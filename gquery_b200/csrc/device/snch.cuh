@@ -175,6 +175,39 @@ __device__ __forceinline__ void load_pair(const DevScene &s, int ref, PairView<D
     }
 }
 
+// Box keys of the traversals that keep the reference's answers up to ties: the distance in
+// 3D, its square in 2D, where the square root is a good part of a visit (1,000,003 queries on
+// 48 polylines 3.37 -> 3.21 ms; the 3D walks, bound by their node bounds and loads, lose 2%).
+//
+// key_limit(r): a box is within r exactly when its key is at most this; in 2D the largest x
+// whose square root rounds to at most r.
+template <int D>
+__device__ __forceinline__ float key_limit(float r) {
+    if (D == 3 || !(r >= 0.f) || r == kInf) return r;  // -1 (a lane without a query), NaN, unlimited
+    float t = fminf(r * r, 3.40282347e38f);
+    while (gq_sqrt(t) > r) t = __int_as_float(__float_as_int(t) - 1);
+    for (;;) {
+        const float u = __int_as_float(__float_as_int(t) + 1);
+        if (u == kInf || !(gq_sqrt(u) <= r)) break;
+        t = u;
+    }
+    return t;
+}
+// Whether the distance of key a is less than that of key b (2D: the rounded square roots,
+// taken only where the squares are within 2^-21).
+template <int D>
+__device__ __forceinline__ bool key_less(float a, float b) {
+    if (D == 3 || !(a < b)) return a < b;
+    return a < b * 0.99999952f || gq_sqrt(a) < gq_sqrt(b);
+}
+template <int D>
+__device__ __forceinline__ float box_key(const float *lo, const float *hi, const float *x) {
+    float u[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) u[k] = fmaxf(fmaxf(lo[k] - x[k], x[k] - hi[k]), 0.f);
+    return D == 2 ? gq_dot2(u[0], u[D - 1], u[0], u[D - 1]) : gq_norm3(u[0], u[1], u[D - 1]);
+}
+
 // Child c of the pair certainly holds no silhouette for x (3D node bound, sil_filter.h;
 // skipping it leaves the reference's answers and the order of its other visits as
 // they are).  The delta form first; with CONE the cone form where it does not decide
