@@ -368,6 +368,9 @@ bool on_host_only(const gq_scene *s) { return s->device < 0; }
 // traversal from this many queries on (measured crossover on B200: ~2^20 for the
 // level-7 benchmark mesh, below it for smaller scenes).
 constexpr int64_t kSilCoherentFrom = 1 << 18;
+// From this many on, queries of the WARP variant are sorted (sorted / in the caller's order: 3D, 301
+// queries 137 / 124 us, 30,011 775 / 714, 60,003 1,813 / 2,009; 2D, 65,521 623 / 574, 200,003 the same).
+constexpr int64_t kSilSortFrom3D = 1 << 15, kSilSortFrom2D = 1 << 17;
 
 // Host trees of a loaded scene, rebuilt on first use: the build is deterministic, so
 // they are the trees the saved device image was flattened from.
@@ -854,7 +857,9 @@ gq_status gq_closest_silhouette(const gq_scene *s, gq_vecs x, const float *r_max
     gq_status st;
     gqd::Tune tune = to_tune(s, GQ_KIND_SILHOUETTE, v);
     const bool middle_first = v == GQ_VARIANT_COHERENT && s->dim == 3;
-    if ((st = prepare_order(s, x, n, opts, cs, scr, &perm, &counter, nullptr, false,
+    // one query per warp: the order only decides which nodes are still in L1
+    const bool any_order = v == GQ_VARIANT_WARP && n < (s->dim == 3 ? kSilSortFrom3D : kSilSortFrom2D);
+    if ((st = prepare_order(s, x, n, opts, cs, scr, &perm, &counter, nullptr, any_order,
                             middle_first && n >= (1 << 18) ? &tune.tiles : nullptr)) != GQ_OK)
         return st;
     cudaError_t e = gqd::launch_sil(s->dev, v, tune, x, r_max, n, perm, *out, counter,

@@ -412,6 +412,7 @@ __device__ __noinline__ void sil_tiles_phase(const DevScene *scenes, int n_scene
                                              const gq_sil_out &sil_out, unsigned long long *counter, int32_t *err) {
     const unsigned lane = threadIdx.x & 31u;
     const int64_t t_sil = (sil.n + 31) / 32;
+    __shared__ uint32_t sink[kBlock];
     snch::Stack stk;
     for (;;) {
         unsigned long long t = 0;
@@ -438,7 +439,7 @@ __device__ __noinline__ void sil_tiles_phase(const DevScene *scenes, int n_scene
             const unsigned m = __ballot_sync(0xffffffffu, alive && sid == s0);
             snch::Lane<D> M = L;
             if (!((m >> lane) & 1u)) M.r = -1.f;
-            pkt::closest_silhouette<D>(scenes[s0], m, M, stk);
+            pkt::closest_silhouette<D, D == 2>(scenes[s0], m, M, stk, sink + (threadIdx.x & ~31u));
             if ((m >> lane) & 1u) L = M;
             todo &= ~m;
         }

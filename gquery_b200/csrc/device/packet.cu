@@ -89,7 +89,10 @@ cudaError_t launch(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const
 // on 1,310,720 triangles: 262,144 5.8 / 7.2 ms, 1,048,576 8.6 / 8.9, 2,097,152 11.5 / 10.7, 8,388,608
 // 23.9 / 19.9; 1,000,003 points near 327,680 triangles 1.25 / 1.55 ms.  Both forms give the
 // same answers bit for bit.
-constexpr int64_t kSparseBelow = 1 << 21;
+// 2D (children brought into L1 ahead, no pairs): 100,003 points on 60,000 segments 842 / 581 us
+// without / with, 2,000,003 on 262,144 3.24 / 2.86 ms, but 1,048,576 on 4,096, whose tree stays in L1
+// anyway, 249 / 260 us, so polylines below 16,384 segments leave it out from 65,536 points on.
+constexpr int64_t kSparseBelow = 1 << 21, kSmallCall2D = 1 << 16, kLargeLine = 1 << 14;
 
 template <int D, int LAYOUT, bool MINFIRST>
 cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const int32_t *perm,
@@ -98,8 +101,8 @@ cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, c
         if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32, true>(s, t, q, n, perm, o, counter, st);
         return launch<D, LAYOUT, MINFIRST, pkt::kPStack, true>(s, t, q, n, perm, o, counter, st);
     }
-    if constexpr (D == 3 && LAYOUT == 0) {
-        if (n < kSparseBelow)
+    if constexpr (LAYOUT == 0) {
+        if (n < kSparseBelow && (D == 3 || n < kSmallCall2D || s.n_prims >= kLargeLine))
             return t.stack == 32
                        ? launch<D, LAYOUT, MINFIRST, 32, false, true>(s, t, q, n, perm, o, counter, st)
                        : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, true>(s, t, q, n, perm, o, counter, st);

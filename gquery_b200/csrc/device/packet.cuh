@@ -323,8 +323,8 @@ __device__ __forceinline__ void leaf(const DevScene &s, int ref, unsigned cmask,
 // 1: quantised 8-wide nodes (3D only).  STK: entries of the caller's stack `stk`; the
 // warp stops with `ovf` set rather than overflow it.
 // COMPACT: the stack of PStack<true> (FP16 keys, one node word per warp).
-// SPARSE (3D, LAYOUT 0): for calls whose time is the latency of a few walks rather than
-// their number: run3's pairs, and the children brought into L1 ahead (+20% on 262,144
+// SPARSE (LAYOUT 0): for calls whose time is the latency of a few walks rather than their
+// number: run3's pairs (3D), and the children brought into L1 ahead (+20% on 262,144 3D
 // points, -5% on 8,388,608).  buf: this warp's LeafBuf in shared memory.
 template <int D, int LAYOUT, bool MINFIRST, int STK = kPStack, bool COMPACT = false, bool SPARSE = false>
 __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, const float *p, float &r, int &idx,
@@ -388,9 +388,11 @@ __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, 
                 // wait for at the next node.
                 const int cref = lane < 16 ? rl : rr;
                 const unsigned w = lane & 15u;
-                const char *from = (const char *)s.pairs + ((int64_t)(cref >= 0 ? cref : cur) * 64 + 4 * w);
-                if (cref < 0 && (cref & 0x40000000) == 0)  // a run: its triangles, at most 288 B
-                    from = (const char *)s.prims + ((int64_t)(cref & 0xffffff) * 48 + min(16 * w, 48 * ((cref >> 24) & 0x3fu) - 4));
+                constexpr unsigned kPair = D == 3 ? 64 : 48, kItem = D == 3 ? 48 : 32;
+                const char *from = (const char *)s.pairs + ((int64_t)(cref >= 0 ? cref : cur) * kPair + min(4 * w, kPair - 4));
+                if (cref < 0 && (cref & 0x40000000) == 0)  // a run: its items, at most 288 B
+                    from = (const char *)s.prims +
+                           ((int64_t)(cref & 0xffffff) * kItem + min(16 * w, kItem * ((cref >> 24) & 0x3fu) - 4));
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sink), "l"(from));
             }
             float a2l = kInf, b2l = kInf, a2r = kInf, b2r = kInf;

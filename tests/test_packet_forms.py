@@ -56,3 +56,17 @@ def test_forms_agree_bitwise_and_with_exact(kind, build):
     # both closest points are formed with a few roundings of the coordinates' size
     tol = 16 * EPS32 * float(np.abs(v).max() + q.abs().max().item())
     assert np.abs(exact["d"].astype(np.float64) - dense["d"][:4099]).max() <= tol
+
+
+@pytest.mark.parametrize("segments,large", [(3, 1 << 16), (300, 1 << 16), (20_000, 1 << 21)])
+def test_2d_forms_agree_bitwise(segments, large):
+    """The 2D walk with and without its children brought ahead: by call size, on small polylines
+    from 65,536 points on, on large ones from 2,097,152."""
+    v, e = W.star_polyline(segments, seed=segments)
+    s = Scene(v, e, 2, device=0, build_snch=False)
+    q = torch.as_tensor(W.uniform_points(large + 5, 2, seed=8)).cuda()
+    fields = ["valid", "p", "n", "t", "d", "prim_id"]
+    whole = to_np(s.closest_point(q, variant="coherent", sort=False))
+    for n in (64, 4096):
+        part = to_np(s.closest_point(q[:n], variant="coherent", sort=False))
+        assert_bitwise(part, {k: whole[k][..., :n] for k in fields}, fields, f"{segments} {n} ")
