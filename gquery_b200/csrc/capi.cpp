@@ -493,7 +493,7 @@ gq_status prepare_order(const gq_scene *s, gq_vecs keys_from, int64_t n, const g
         if ((size_t)opts->scratch_bytes < need) return fail(GQ_ERR_INVALID, "scratch buffer too small");
         scr.p = opts->scratch;
     } else {
-        cudaError_t e = scratch_alloc(s, &scr.p, need, st);
+        cudaError_t e = scratch_alloc(s, &scr.p, any_order ? kCounterBytes : need, st);
         if (e != cudaSuccess) return fail(GQ_ERR_NOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
         scr.owned = true;
         scr.st = st;
