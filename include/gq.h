@@ -130,7 +130,8 @@ typedef struct {
 
 typedef struct {
     int32_t variant;        /* GQ_VARIANT_* */
-    int32_t sort;           /* 1: reorder queries along a space-filling curve before traversal (gq_query_order) */
+    int32_t sort;           /* 1: reorder queries along a space-filling curve before traversal (gq_query_order) where
+                               that pays; calls whose answers do not depend on the order may keep the caller's */
     const int32_t *order;   /* optional device permutation from gq_query_order(); replaces `sort` */
     void *scratch;          /* optional device scratch (see gq_query_scratch_bytes); NULL = stream-ordered allocation */
     int64_t scratch_bytes;
