@@ -448,6 +448,7 @@ __device__ __noinline__ void sil_tiles_phase(const DevScene *scenes, int n_scene
             put_sil<D>(sil_out, sil.n, qi, alive && L.found && !L.ovf, L.bp, L.bd, L.bid);
         }
     }
+    if (D == 2) pkt::copies_done();
 }
 
 // Silhouettes, one lane per query in the reference's order.

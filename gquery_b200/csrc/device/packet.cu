@@ -57,6 +57,7 @@ __global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q,
                 cp2_record(s.prims, idx, (idx >= 0) && !ovf, p[0], p[D - 1], o, n, qi);
         }
     }
+    if (SPARSE) pkt::copies_done();
 }
 
 template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT = false, bool SPARSE = false>

@@ -96,6 +96,10 @@ __device__ __forceinline__ float sqrt_approx(float x) {
     return y;
 }
 
+// Ends the asynchronous copies that the walks started to bring nodes into L1: shared memory
+// may go to another block, or be used for something else, only after this.
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // squared distances from p to the nearest / farthest point of a box
 template <int D>
 __device__ __forceinline__ void box_sq(const float *lo, const float *hi, const float *p, float &a2, float &b2) {
