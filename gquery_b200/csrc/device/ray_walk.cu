@@ -86,7 +86,8 @@ cudaError_t launch(const DevScene &s, gq_vecs x, gq_vecs v, const float *r_max, 
 cudaError_t launch_ray_walk(const DevScene &s, gq_vecs x, gq_vecs v, const float *r_max, int64_t n, const int32_t *perm,
                             const gq_ray_out &o, unsigned long long *counter, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    if (!s.wnodes || !counter) return cudaErrorInvalidValue;
+    // a tree that is one leaf has no nodes: its root is the leaf
+    if ((!s.wnodes && s.wroot_ref >= 0) || !counter) return cudaErrorInvalidValue;
     return s.dim == 3 ? launch<3>(s, x, v, r_max, n, perm, o, counter, st)
                       : launch<2>(s, x, v, r_max, n, perm, o, counter, st);
 }
