@@ -18,7 +18,8 @@
 // the reference's.  The nearest hit does not depend on the order of the visits unless two
 // items are hit at exactly the same t; such a ray (2 of 8,388,608 on the benchmark) is
 // walked again by the other walk, whose order picks the winner: the answers are that
-// walk's bit for bit.
+// walk's bit for bit.  So is a ray whose products could leave the range in which the margins
+// hold (init()).
 #pragma once
 
 #include "prim.cuh"
@@ -38,7 +39,7 @@ struct Lane {
     float iv[D], on[D], of[D];  // 1 / direction; -p iv moved down / up by eps |iv|
     float r;                    // r_max, then the nearest hit
     int idx, cur, sp;
-    bool tie, ovf;
+    bool again, ovf;            // again: the other walk answers this ray
 };
 
 // Both planes of one axis: the near one into tn, the far one into tf.
@@ -66,12 +67,20 @@ __device__ __forceinline__ void init(const DevScene &s, Lane<D> &L, const gq_vec
         pmax = fmaxf(pmax, fabsf(L.p[k]));
         vmax = fmaxf(vmax, fabsf(L.v[k]));
     }
-    const float eps = (pmax + s.coord_bound) * 9.5367432e-07f;  // 2^-20
+    const float size = pmax + s.coord_bound, eps = size * 9.5367432e-07f;  // 2^-20
+    bool tame = true;
 #pragma unroll
     for (int k = 0; k < D; ++k) {
         // a component below 1e-12 of the largest moves the ray by less than eps over any
         // distance that matters, and would overflow the products
-        L.iv[k] = __fdividef(1.f, copysignf(fmaxf(fabsf(L.v[k]), vmax * 1e-12f), L.v[k]));
+        L.iv[k] = gq_div(1.f, copysignf(fmaxf(fabsf(L.v[k]), vmax * 1e-12f), L.v[k]));
+        // Parameters t are at most some 2^9 times size / |direction| (a node's origin lies 2^15
+        // of its steps low), the margin is 2^-20 of it.  From 2^-110 to 2^110 neither
+        // overflows, and the margin is above 2^5 times what subnormal products lose.  Outside,
+        // and where a component is infinite (iv = 0, and with it every t), boxes could be lost or
+        // none left out.
+        const float t = size * fabsf(L.iv[k]);
+        tame = tame && t >= 7.7037198e-34f && t <= 1.2980742e33f;
         const float o = -(L.p[k] * L.iv[k]), e = eps * fabsf(L.iv[k]);
         L.on[k] = o - e;
         L.of[k] = o + e;
@@ -79,11 +88,11 @@ __device__ __forceinline__ void init(const DevScene &s, Lane<D> &L, const gq_vec
     L.r = rmax_in ? rmax_in[qi] : kInf;
     L.idx = -1;
     L.sp = -1;
-    L.tie = false;
+    L.again = !tame && vmax > 0.f;
     L.ovf = false;
     float tn, tf;
     slab<D>(L, s.root_lo, s.root_hi, tn, tf);
-    bool enter = vmax > 0.f && tn <= tf;  // a ray without a direction hits nothing
+    bool enter = tame && tn <= tf;  // a ray without a direction hits nothing
     if (enter) {
         // the reference's own test of the root box (bvh.py:209-216), which decides
         float t_root;
@@ -219,9 +228,9 @@ __device__ __forceinline__ void take(Lane<D> &L, float key, int j) {
     if (key < L.r) {
         L.r = key;
         L.idx = j;
-        L.tie = false;
+        L.again = false;
     } else if (key == L.r && L.idx >= 0) {
-        L.tie = true;
+        L.again = true;
     }
 }
 
@@ -291,22 +300,28 @@ __device__ __forceinline__ void leaves(const void *prims, Lane<D> &L, const int2
     }
 }
 
-// The winner of a ray with an exact tie: the walk over the 8-wide nodes.
+// A ray with an exact tie or outside this walk's range: the other walk over the 8-wide nodes.
+// Returns its primitive and the bits of its t, -2 after a stack overflow.
 template <int D>
-__device__ __noinline__ int tie_winner(const DevScene &s, const gq_vecs &a, const gq_vecs &b, const float *rmax_in,
-                                       int64_t qi) {
+__device__ __noinline__ int2 other_walk(const DevScene &s, const gq_vecs &a, const gq_vecs &b, const float *rmax_in,
+                                        int64_t qi) {
     trav::Stack<true> stk;
     trav::Lane<D, true, true> W;
     trav::lane_init(s, W, a, b, rmax_in, qi);
     while (!trav::lane_run<D, true, true, 0>(s, W, stk, 1 << 30)) {
     }
-    return W.ovf ? -1 : W.idx;
+    return make_int2(W.ovf ? -2 : W.idx, fbits(W.r));
 }
 
 template <int D>
 __device__ __forceinline__ void finish(const DevScene &s, Lane<D> &L, const gq_vecs &a, const gq_vecs &b,
                                        const float *rmax_in, int64_t qi, int64_t n, const gq_ray_out &o) {
-    if (L.tie) L.idx = tie_winner<D>(s, a, b, rmax_in, qi);
+    if (L.again) {
+        const int2 w = other_walk<D>(s, a, b, rmax_in, qi);
+        L.idx = w.x;
+        L.r = __int_as_float(w.y);
+        L.ovf = w.x == -2;
+    }
     if (L.ovf && s.err) atomicOr(s.err, GQ_DEVERR_STACK);
     const bool found = L.idx >= 0 && !L.ovf;
     if (D == 3)
