@@ -223,6 +223,8 @@ __device__ __forceinline__ float item_ray(const void *prims, int j, const float 
     return seg_ray(p[0], p[D - 1], v[0], v[D - 1], a.x, a.y, a.z, a.w);
 }
 
+// The nearest item (j at t = key) of a leaf or run.  Both walks test its items in order and keep
+// the first of equals; only an equal item of another leaf (L.idx) leaves the order open.
 template <int D>
 __device__ __forceinline__ void take(Lane<D> &L, float key, int j) {
     if (key < L.r) {
@@ -245,7 +247,7 @@ struct LeafBuf {
 // A run holds up to six items and the rays that skim a surface meet hundreds of them
 // one after another, which is what a call of few rays waits for; so the pairs (item, lane) of all
 // waiting lanes are listed in shared memory and every lane of the warp tests one.
-// Each ray's lane then takes its keys in the items' order.
+// Each ray's lane then takes the first of its smallest keys.
 // MANY: the rays may be of different scenes (each lane passes its scene's items).
 template <int D, bool MANY>
 __device__ __forceinline__ void leaves(const void *prims, Lane<D> &L, const int2 *stk, LeafBuf &buf) {
@@ -282,10 +284,17 @@ __device__ __forceinline__ void leaves(const void *prims, Lane<D> &L, const int2
         if (k < total) buf.key[k] = item_ray<D>(items, j, p, v, last);
     }
     __syncwarp();
-    int base = 0;
+    float key = kInf;  // nearest of the leaf
+    int at = first, base = 0;
 #pragma unroll
     for (int t = 0; t < GQ_COLLAPSE_MAX; ++t) {
-        if (t < count) take<D>(L, buf.key[base + __popc(m[t] & below)], first + t);
+        if (t < count) {
+            const float k = buf.key[base + __popc(m[t] & below)];
+            if (k < key) {
+                key = k;
+                at = first + t;
+            }
+        }
         base += __popc(m[t]);
     }
     __syncwarp();  // the buffer is free again
@@ -293,9 +302,14 @@ __device__ __forceinline__ void leaves(const void *prims, Lane<D> &L, const int2
         if (!run)
             for (int j = first;; ++j) {
                 bool last;
-                take<D>(L, item_ray<D>(prims, j, L.p, L.v, last), j);
+                const float k = item_ray<D>(prims, j, L.p, L.v, last);
+                if (k < key) {
+                    key = k;
+                    at = j;
+                }
                 if (last) break;
             }
+        take<D>(L, key, at);
         pop<D>(L, stk);
     }
 }
