@@ -13,7 +13,10 @@
 // Pruning keeps every box within eps (2^-19 of the coordinates' size) of the radius, so all
 // candidates for the minimum are met.  Where the reference's own pruning could have
 // decided otherwise by a rounding (a box's farthest point within eps of the answer, or a
-// leaf box farther than its primitive), the query is walked again in the plain order.
+// leaf box farther than its primitive), the query is walked again in the plain order.  A
+// query so far away that eps spans the scene, or without a finite distance, ends up there
+// as soon as that shows: no answer is nearer than the root box (16 points a million radii from
+// 327,680 triangles 15.9 -> 0.62 ms).
 #include <algorithm>
 
 #include "prim.cuh"
@@ -75,12 +78,28 @@ __global__ void __launch_bounds__(32) k_cp_few(DevScene s, gq_vecs q, int64_t n,
     unsigned long long path = ~0ull;  // and that one's place in the reference's order
     bool odd = false;              // a leaf box farther than that primitive
     float far = kInf;              // smallest farthest-point distance of any box
+    float sure;                    // an answer may stand only while that is above this
+    {
+        float dmin, dmax, sum = 0.f;
+        if (D == 3)
+            box_dist3(s.root_lo[0], s.root_lo[1], s.root_lo[2], s.root_hi[0], s.root_hi[1], s.root_hi[2], p[0], p[1],
+                      p[D - 1], dmin, dmax);
+        else
+            box_dist2(s.root_lo[0], s.root_lo[1], s.root_hi[0], s.root_hi[1], p[0], p[D - 1], dmin, dmax);
+#pragma unroll
+        for (int k = 0; k < D; ++k) sum += p[k];
+        sure = sum == sum ? dmin + eps : kInf;  // a NaN is ignored by the box tests
+    }
     float R = kInf;                // the warp's radius
     int sp = 1;
     if (lane == 0) stk[0] = Entry{s.root_ref, 0.f, 1ull << 63};
     __syncwarp();
-    bool full = false;
+    bool full = false;  // left to the plain walk
     while (sp > 0) {
+        if (__any_sync(0xffffffffu, !(far > sure))) {
+            full = true;
+            break;
+        }
         const int take = (sp + 32 <= kStackF - kReserveF) ? min(sp, 32) : 1;
         const bool mine = (int)lane < take;
         Entry e{0, 0.f, 0ull};
