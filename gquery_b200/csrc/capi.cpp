@@ -80,23 +80,23 @@ namespace {
 
 void default_tuning(gq_scene *s);
 
-// Bounding cylinders of the triangles and of the pair records' runs (layout.h), computed
-// on the device from the uploaded records; the caller has selected the scene's device.
+// Bounding cylinders of the pair records' runs (layout.h), computed on the device from the
+// uploaded records, with a place for every triangle (32 B each, also where a tree has no runs:
+// a record read from a file may name any); the caller has selected the scene's device.
 gq_status add_cylinders(gq_scene *s) {
     if (s->dim != 3 || s->np < 1) return GQ_OK;
     gqd::DevScene &d = s->dev;
-    const size_t bytes = 2 * sizeof(gq_cyl_t) * (size_t)s->np;
+    const size_t bytes = sizeof(gq_cyl_t) * (size_t)s->np;
     void *p = nullptr;
     cudaError_t e = cudaMalloc(&p, bytes);
     if (e != cudaSuccess) return fail(GQ_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     s->allocs.push_back(p);
     s->device_bytes += (int64_t)bytes;
-    gq_cyl_t *tri = (gq_cyl_t *)p, *run = tri + s->np;
-    e = gqd::build_cylinders(d, (int64_t)(s->image_bytes[0] / sizeof(gq_pair3_t)), tri, run);
+    d.run_cyl = (gq_cyl_t *)p;
+    d.has_runs = !s->gpu_built;
+    e = gqd::build_cylinders(d, (int64_t)(s->image_bytes[0] / sizeof(gq_pair3_t)), (gq_cyl_t *)p);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) return fail_cuda(e, "bounding cylinders");
-    d.tri_cyl = tri;
-    d.run_cyl = run;
     return GQ_OK;
 }
 

@@ -15,10 +15,10 @@ __device__ __forceinline__ float qget(const gq_vecs &v, int64_t i, int k) {
     return v.ptr[(int64_t)k * v.comp_stride + i * v.elem_stride];
 }
 
-// Registers: 56 keep 36 warps on an SM (8,388,608 points: 48 / 56 / 64 registers 20.4-21.6 /
-// 19.4-20.2 / 22.4 ms); the sparse form needs 64 for its loops and is bound by latency.
-template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT, bool SPARSE>
-__global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q, int64_t n, const int32_t *perm, const int32_t *tiles,
+// Registers: 56 keep 36 warps on an SM; the form that fetches ahead needs 64 for its loops and is
+// bound by latency.
+template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT, int FORM>
+__global__ void __maxnreg__(FORM == 2 ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q, int64_t n, const int32_t *perm, const int32_t *tiles,
                                                          gq_cp_out o, unsigned long long *counter) {
     const unsigned lane = threadIdx.x & 31u;
     // (ref, this lane's key) per entry; refs are the same in every lane
@@ -32,7 +32,7 @@ __global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q,
             return pkt::PStack<false>(plain);
     }();
     extern __shared__ pkt::LeafBuf leaf_buf[];
-    pkt::LeafBuf *buf = SPARSE ? leaf_buf + (threadIdx.x >> 5) : nullptr;
+    pkt::LeafBuf *buf = FORM ? leaf_buf + (threadIdx.x >> 5) : nullptr;
     for (;;) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(counter, 32ull);
@@ -47,7 +47,7 @@ __global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q,
         float r = kInf;
         int idx = -1;
         bool ovf = false;
-        pkt::closest_point<D, LAYOUT, MINFIRST, STK, COMPACT, SPARSE>(s, __ballot_sync(0xffffffffu, alive), p, r, idx, ovf,
+        pkt::closest_point<D, LAYOUT, MINFIRST, STK, COMPACT, FORM>(s, __ballot_sync(0xffffffffu, alive), p, r, idx, ovf,
                                                              stk, buf);
         if (ovf && lane == 0 && s.err) atomicOr(s.err, GQ_DEVERR_STACK);
         if (alive) {
@@ -57,43 +57,46 @@ __global__ void __maxnreg__(SPARSE ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q,
                 cp2_record(s.prims, idx, (idx >= 0) && !ovf, p[0], p[D - 1], o, n, qi);
         }
     }
-    if (SPARSE) pkt::copies_done();
+    if (FORM == 2) pkt::copies_done();
 }
 
-template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT = false, bool SPARSE = false>
+template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT = false, int FORM = 0>
 cudaError_t launch(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const int32_t *perm, const gq_cp_out &o,
                    unsigned long long *counter, cudaStream_t st) {
     static int bps[3] = {0, 0, 0}, n_sm = 0;
     int block = t.block, slot = block_slot(block);
     if (slot < 0) slot = 1, block = 128;
-    const size_t smem = SPARSE ? (size_t)(block / 32) * sizeof(pkt::LeafBuf) : 0;
+    const size_t smem = FORM ? (size_t)(block / 32) * sizeof(pkt::LeafBuf) : 0;
     if (!bps[slot]) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, SPARSE>, block, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, FORM>, block, smem);
         bps[slot] = b < 1 ? 1 : b;
     }
     const int64_t warps = (n + 31) / 32;
     const int64_t want = std::min<int64_t>((int64_t)bps[slot] * n_sm, (warps * 32 + block - 1) / block);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, SPARSE><<<dim3((unsigned)want), block, smem, st>>>(s, q, n, perm, t.tiles, o,
+    k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, FORM><<<dim3((unsigned)want), block, smem, st>>>(s, q, n, perm, t.tiles, o,
                                                                                                    counter);
     return cudaGetLastError();
 }
 
-// Calls of fewer queries run the sparse form of the walk (packet.cuh), whose time is the
-// latency of the heaviest tiles; from here on the GPU has about fifteen tiles per
-// resident warp and the form with more warps wins.  Sparse against dense form, uniform points
-// on 1,310,720 triangles: 262,144 5.8 / 7.2 ms, 1,048,576 8.6 / 8.9, 2,097,152 11.5 / 10.7, 8,388,608
-// 23.9 / 19.9; 1,000,003 points near 327,680 triangles 1.25 / 1.55 ms.  Both forms give the
-// same answers bit for bit.
-// 2D (children brought into L1 ahead, no pairs): 100,003 points on 60,000 segments 842 / 581 us
-// without / with, 2,000,003 on 262,144 3.24 / 2.86 ms, but 1,048,576 on 4,096, whose tree stays in L1
-// anyway, 249 / 260 us, so polylines below 16,384 segments leave it out from 65,536 points on.
-constexpr int64_t kSparseBelow = 1 << 21, kSmallCall2D = 1 << 16, kLargeLine = 1 << 14;
+// Calls of fewer queries bring children into L1 ahead (packet.cuh): their time is the latency of
+// the heaviest tiles; from here on the GPU has some thirty tiles per resident warp and the
+// form with more warps wins.  Without / with, uniform points on 1,310,720 triangles and on a tube
+// of 320,000 slivers: 2,097,157 10.0 / 8.8 and 22.0 / 21.2 ms, 4,194,304 12.4 / 12.1 and 24.6 / 26.5,
+// 6,000,000 14.4 / 14.8 and 30.5 / 32.6, 8,388,608 17.5 / 19.5 and 39.4 / 41.7.
+// Device-built trees, one triangle per leaf, leave it out earlier: 327,680 curved and 200,000
+// scattered triangles, 262,144 points 7.3 / 6.7 and 0.55 / 0.55 ms, 1,048,576 8.4 / 8.0 and 0.69 / 0.80.
+// All forms give the same answers bit for bit.
+// 2D (no pairs): 100,003 points on 60,000 segments 842 / 581 us without / with, 2,000,003 on 262,144
+// 3.24 / 2.86 ms, but 1,048,576 on 4,096, whose tree stays in L1 anyway, 249 / 260 us, so
+// polylines below 16,384 segments leave it out from 65,536 points on, the others from 2,097,152.
+constexpr int64_t kAheadBelow3D = 1 << 22, kAheadNoRuns = 1 << 19;
+constexpr int64_t kAheadBelow2D = 1 << 21, kSmallCall2D = 1 << 16, kLargeLine = 1 << 14;
 
 template <int D, int LAYOUT, bool MINFIRST>
 cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const int32_t *perm,
@@ -103,10 +106,14 @@ cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, c
         return launch<D, LAYOUT, MINFIRST, pkt::kPStack, true>(s, t, q, n, perm, o, counter, st);
     }
     if constexpr (LAYOUT == 0) {
-        if (n < kSparseBelow && (D == 3 || n < kSmallCall2D || s.n_prims >= kLargeLine))
-            return t.stack == 32
-                       ? launch<D, LAYOUT, MINFIRST, 32, false, true>(s, t, q, n, perm, o, counter, st)
-                       : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, true>(s, t, q, n, perm, o, counter, st);
+        const bool ahead = D == 3 ? n < (s.has_runs ? kAheadBelow3D : kAheadNoRuns)
+                                  : n < (s.n_prims >= kLargeLine ? kAheadBelow2D : kSmallCall2D);
+        if (ahead)
+            return t.stack == 32 ? launch<D, LAYOUT, MINFIRST, 32, false, 2>(s, t, q, n, perm, o, counter, st)
+                                 : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, 2>(s, t, q, n, perm, o, counter, st);
+        if constexpr (D == 3)
+            return t.stack == 32 ? launch<D, LAYOUT, MINFIRST, 32, false, 1>(s, t, q, n, perm, o, counter, st)
+                                 : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, 1>(s, t, q, n, perm, o, counter, st);
     }
     if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32>(s, t, q, n, perm, o, counter, st);
     return launch<D, LAYOUT, MINFIRST, pkt::kPStack>(s, t, q, n, perm, o, counter, st);
@@ -178,11 +185,6 @@ __device__ void cylinder_of(const gq_tri_t *prims, int64_t first, int count, gq_
     out.half = ok ? __double2float_ru(half + slack) : kInf;
 }
 
-__global__ void __launch_bounds__(128) k_tri_cyl(const gq_tri_t *prims, int64_t n, gq_cyl_t *out) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) cylinder_of(prims, i, 1, out[i]);
-}
-
 // The walk meets the largest runs only: the two runs of a pair that is itself inside a run
 // are left out (they may start at the same triangle as the run around them).
 __global__ void __launch_bounds__(128) k_run_cyl(const gq_pair3_t *pairs, int64_t n, int32_t root, const gq_tri_t *prims,
@@ -199,15 +201,11 @@ __global__ void __launch_bounds__(128) k_run_cyl(const gq_pair3_t *pairs, int64_
 
 }  // namespace
 
-cudaError_t build_cylinders(const DevScene &s, int64_t n_pairs, gq_cyl_t *tri_cyl, gq_cyl_t *run_cyl) {
-    const gq_tri_t *prims = static_cast<const gq_tri_t *>(s.prims);
-    if (s.n_prims > 0)
-        k_tri_cyl<<<dim3((unsigned)((s.n_prims + 127) / 128)), 128>>>(prims, s.n_prims, tri_cyl);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+cudaError_t build_cylinders(const DevScene &s, int64_t n_pairs, gq_cyl_t *run_cyl) {
     if (n_pairs > 0)
         k_run_cyl<<<dim3((unsigned)((2 * n_pairs + 127) / 128)), 128>>>(
-            static_cast<const gq_pair3_t *>(s.pairs), n_pairs, s.root_ref, prims, s.n_prims, run_cyl);
+            static_cast<const gq_pair3_t *>(s.pairs), n_pairs, s.root_ref, static_cast<const gq_tri_t *>(s.prims),
+            s.n_prims, run_cyl);
     return cudaGetLastError();
 }
 

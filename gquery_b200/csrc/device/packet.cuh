@@ -181,9 +181,9 @@ __device__ __forceinline__ float tri_key(float px, float py, float pz, float ax,
     return gq_dot3(ex, ey, ez, ex, ey, ez);
 }
 
-// Pairs of a triangle and a lane that a sparse walk tests without bounds: two rounds of the
-// warp (32 / 64 / 96: 250,007 points near a 327,680-triangle surface 786 / 743 / 724 us,
-// 8,388,608 uniform points on 1,310,720 triangles 22.4 / 22.7 / 23.9 ms).
+// Pairs of a triangle and a lane that are tested side by side: two rounds of the warp (32 / 64 /
+// 96: 250,007 points near a 327,680-triangle surface 786 / 743 / 724 us, 8,388,608 uniform points
+// on 1,310,720 triangles 22.4 / 22.7 / 23.9 ms).
 constexpr int kRunPairs = 64;
 // Shared memory of one warp for the (triangle of a run, lane) pairs of leaf().
 struct LeafBuf {
@@ -193,33 +193,63 @@ struct LeafBuf {
 };
 static_assert(GQ_COLLAPSE_MAX <= 8, "a pair of leaf() fits a byte");
 
+// Triangle j for the lanes with `act`; whether it is its leaf's last.
+__device__ __forceinline__ bool tri_test(const DevScene &s, int j, bool act, const float *p, float &r, int &idx) {
+    const float4 t0 = ldg4(s.prims, 3 * (int64_t)j), t1 = ldg4(s.prims, 3 * (int64_t)j + 1),
+                 t2 = ldg4(s.prims, 3 * (int64_t)j + 2);
+    if (act) {
+        float pt[3], u, v;
+        tri_closest<true>(p[0], p[1], p[2], t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x, pt, &u, &v);
+        const float ex = p[0] - pt[0], ey = p[1] - pt[1], ez = p[2] - pt[2];
+        const float key = gq_dot3(ex, ey, ez, ex, ey, ez);
+        if (key < r) {
+            r = key;
+            idx = j;
+        }
+    }
+    return (fbits(t2.z) & GQ_ITEM_LAST) != 0;
+}
+
 // A run of at most GQ_COLLAPSE_MAX triangles from `first`, for the lanes in cmask.
 //
 // A triangle test costs about 100 instructions and nearly none improves a lane: of 584 per
 // tile of 32 queries (8,388,608 uniform points on 1,310,720 triangles; counts of a model of
-// the walk) 32 do.
+// the walk) 32 do.  So the run's cylinder (about 20 instructions) comes first: it leaves out 72
+// of the tile's 126 runs, and most lanes of the others.
 //
-// SPARSE, few lanes (at most kRunPairs pairs of a triangle and a lane): the lanes that need a
-// run are few where queries are sparse (8 of 32 near a surface, 4 for 2,003 points).  The
-// pairs are listed in shared memory, every lane of the warp tests one, and each query's
-// lane then takes its keys in the triangles' order.
+// FORM > 0: at most kRunPairs pairs of a triangle and a lane that is left (few lanes need a run
+// where queries are sparse: 8 of 32 near a surface, 4 for 2,003 points) are listed in shared
+// memory, every lane of the warp tests one, and each query's lane then takes its keys in the
+// triangles' order.  Otherwise the lanes test the triangles one by one.  FORM 2, bound by
+// latency, asks the cylinder only where there are more pairs (cylinder first / pairs first:
+// 16,384 points on 327,680 curved triangles 2.16 / 2.31 ms, on 318,402 coplanar ones 455 / 426 us).
 //
-// Otherwise the run's cylinder and then each triangle's disc (about 20 instructions each)
-// are tested first, and a triangle is left out when no lane can improve: 72 of 126 runs, and
-// 472 of the 584 triangles in all.
+// FORM 1, without / with the cylinder before the pairs: 2,097,157 points near 327,680 triangles 7.7 /
+// 6.6 ms, 8,388,608 uniform on 1,310,720 20.4 / 17.5; on a tube of 320,000 slivers, which bound nothing,
+// 21.9 / 22.0 and 43.1 / 39.4.  A disc per triangle before its test, in place of the pairs: 8.9, 18.2,
+// 30.6 and 47.6 ms.
 //
 // A test that is left out would have left every lane's radius and winner as they are
 // (cyl_limit), and the pairs are taken in the order of the plain loop, so the walk
 // and its answers are those of testing every triangle, ties included.
 // RUNCYL: the run is a pair record's (run_cyl holds its cylinder).
-template <bool RUNCYL, bool SPARSE>
+template <bool RUNCYL, int FORM>
 __device__ __forceinline__ void run3(const DevScene &s, int first, int count, unsigned cmask, const float *p, float eps,
                                      float &r, int &idx, LeafBuf *buf) {
     const unsigned lane = threadIdx.x & 31u;
-    const bool act = (cmask >> lane) & 1u;
-    const int lanes = __popc(cmask), total = lanes * count;
-    if (SPARSE && total <= kRunPairs) {
-        const int rank = __popc(cmask & ((1u << lane) - 1u));
+    unsigned need = cmask;
+    if (RUNCYL && !(FORM == 2 && __popc(cmask) * count <= kRunPairs)) {
+        const float4 c = ldg4(s.run_cyl, 2 * (int64_t)first), n = ldg4(s.run_cyl, 2 * (int64_t)first + 1);
+        if (c.w < kInf) {
+            need = __ballot_sync(0xffffffffu, ((cmask >> lane) & 1u) &&
+                                                  !(cyl_bound(c, n, p[0], p[1], p[2]) > cyl_limit(r, eps)));
+            if (!need) return;
+        }
+    }
+    const bool act = (need >> lane) & 1u;
+    const int lanes = __popc(need), total = lanes * count;
+    if (FORM && total <= kRunPairs) {
+        const int rank = __popc(need & ((1u << lane) - 1u));
         if (act)
             for (int t = 0; t < count; ++t) buf->pair[t * lanes + rank] = (uint8_t)(t << 5 | lane);
         __syncwarp();
@@ -246,33 +276,11 @@ __device__ __forceinline__ void run3(const DevScene &s, int first, int count, un
         __syncwarp();  // the buffer is free again
         return;
     }
-    float lim = cyl_limit(r, eps);
-    if (RUNCYL) {
-        const float4 c = ldg4(s.run_cyl, 2 * (int64_t)first), n = ldg4(s.run_cyl, 2 * (int64_t)first + 1);
-        if (!__any_sync(0xffffffffu, act && !(cyl_bound(c, n, p[0], p[1], p[2]) > lim))) return;
-    }
-    for (int j = first; j < first + count; ++j) {
-        const float4 c = ldg4(s.tri_cyl, 2 * (int64_t)j), n = ldg4(s.tri_cyl, 2 * (int64_t)j + 1);
-        const bool need = act && !(cyl_bound(c, n, p[0], p[1], p[2]) > lim);
-        if (!__any_sync(0xffffffffu, need)) continue;
-        const float4 t0 = ldg4(s.prims, 3 * (int64_t)j), t1 = ldg4(s.prims, 3 * (int64_t)j + 1),
-                     t2 = ldg4(s.prims, 3 * (int64_t)j + 2);
-        if (need) {
-            float pt[3], u, v;
-            tri_closest<true>(p[0], p[1], p[2], t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x, pt, &u, &v);
-            const float ex = p[0] - pt[0], ey = p[1] - pt[1], ez = p[2] - pt[2];
-            const float key = gq_dot3(ex, ey, ez, ex, ey, ez);
-            if (key < r) {
-                r = key;
-                idx = j;
-                lim = cyl_limit(r, eps);
-            }
-        }
-    }
+    for (int j = first; j < first + count; ++j) tri_test(s, j, act, p, r, idx);
 }
 
 // Leaf: every lane that needs it (cmask) tests the leaf's items against its query.
-template <int D, bool RUNCYL, bool SPARSE>
+template <int D, bool RUNCYL, int FORM>
 __device__ __forceinline__ void leaf(const DevScene &s, int ref, unsigned cmask, const float *p, float eps, float &r,
                                      int &idx, LeafBuf *buf) {
     const bool act = (cmask >> (threadIdx.x & 31u)) & 1u;
@@ -283,24 +291,13 @@ __device__ __forceinline__ void leaf(const DevScene &s, int ref, unsigned cmask,
     const int end = run ? j + ((ref >> 24) & 0x3f) : 0;
     if (run && end == j) return;  // an empty run (INT32_MIN, an unused wide slot): nothing to test
     if (D == 3 && run) {
-        run3<RUNCYL, SPARSE>(s, j, end - j, cmask, p, eps, r, idx, buf);
+        run3<RUNCYL, FORM>(s, j, end - j, cmask, p, eps, r, idx, buf);
         return;
     }
     for (;;) {
         bool last;
         if (D == 3) {
-            // a leaf of more than GQ_COLLAPSE_MAX triangles, or a device-built tree's
-            const float4 c = ldg4(s.tri_cyl, 2 * (int64_t)j), n = ldg4(s.tri_cyl, 2 * (int64_t)j + 1);
-            const float4 t0 = ldg4(s.prims, 3 * (int64_t)j), t1 = ldg4(s.prims, 3 * (int64_t)j + 1),
-                         t2 = ldg4(s.prims, 3 * (int64_t)j + 2);
-            last = (fbits(t2.z) & GQ_ITEM_LAST) != 0;
-            if (act && !(cyl_bound(c, n, p[0], p[1], p[D - 1]) > cyl_limit(r, eps))) {
-                const float key = tri_key(p[0], p[1], p[D - 1], t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x);
-                if (key < r) {
-                    r = key;
-                    idx = j;
-                }
-            }
+            last = tri_test(s, j, act, p, r, idx);  // a leaf of more than GQ_COLLAPSE_MAX triangles, or a device-built tree's
         } else {
             const float4 a = ldg4(s.prims, 2 * (int64_t)j);
             const int4 f = __ldg(reinterpret_cast<const int4 *>(s.prims) + 2 * (int64_t)j + 1);
@@ -327,10 +324,10 @@ __device__ __forceinline__ void leaf(const DevScene &s, int ref, unsigned cmask,
 // 1: quantised 8-wide nodes (3D only).  STK: entries of the caller's stack `stk`; the
 // warp stops with `ovf` set rather than overflow it.
 // COMPACT: the stack of PStack<true> (FP16 keys, one node word per warp).
-// SPARSE (LAYOUT 0): for calls whose time is the latency of a few walks rather than their
-// number: run3's pairs (3D), and the children brought into L1 ahead (+20% on 262,144 3D
-// points, -5% on 8,388,608).  buf: this warp's LeafBuf in shared memory.
-template <int D, int LAYOUT, bool MINFIRST, int STK = kPStack, bool COMPACT = false, bool SPARSE = false>
+// FORM (LAYOUT 0): 1 run3's pairs (3D); 2 those and the children brought into L1 ahead, for calls
+// whose time is the latency of a few walks rather than their number.  buf: this warp's
+// LeafBuf in shared memory.
+template <int D, int LAYOUT, bool MINFIRST, int STK = kPStack, bool COMPACT = false, int FORM = 0>
 __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, const float *p, float &r, int &idx,
                                               bool &ovf, PStack<COMPACT> stk, LeafBuf *buf = nullptr) {
     const unsigned lane = threadIdx.x & 31u;
@@ -338,7 +335,7 @@ __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, 
     if (!mine) r = 0.f;  // never needs a node
     float eps = 0.f;
     if (D == 3) eps = (fmaxf(fmaxf(fabsf(p[0]), fabsf(p[1])), fabsf(p[D - 1])) + s.coord_bound) * 1.9073486e-06f;  // 2^-19
-    const unsigned sink = SPARSE ? (unsigned)__cvta_generic_to_shared(&buf->sink[lane]) : 0u;
+    const unsigned sink = FORM == 2 ? (unsigned)__cvta_generic_to_shared(&buf->sink[lane]) : 0u;
     int cur = LAYOUT ? s.wroot_ref : s.root_ref;
     unsigned cmask = mask;
     int sp = -1;
@@ -361,7 +358,7 @@ __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, 
         }
         const bool act = (cmask >> lane) & 1u;
         if (cur < 0) {
-            leaf<D, LAYOUT == 0, SPARSE>(s, cur, cmask, p, eps, r, idx, buf);
+            leaf<D, LAYOUT == 0, FORM>(s, cur, cmask, p, eps, r, idx, buf);
             cur = kNone;
             continue;
         }
@@ -385,7 +382,7 @@ __device__ __forceinline__ void closest_point(const DevScene &s, unsigned mask, 
                 rl = rf.z ? (int)(0x80000000u | (unsigned)rf.z) : rf.x;
                 rr = rf.w ? (int)(0x80000000u | (unsigned)rf.w) : rf.y;
             }
-            if (SPARSE) {
+            if (FORM == 2) {
                 // Bring what a visit of either child reads first into L1 while the boxes are
                 // tested: half a warp per child, 4 bytes a lane to a place nobody reads.  An
                 // asynchronous copy needs no destination register, which a load would have to

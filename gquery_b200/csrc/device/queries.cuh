@@ -14,7 +14,7 @@ struct DevScene {
     const void *pairs;   // gq_pair2_t / gq_pair3_t
     const void *prims;   // gq_seg_t / gq_tri_t
     const gq_tsph_t *spheres;  // 3D: bounding sphere per ordered triangle
-    const gq_cyl_t *tri_cyl = nullptr;  // 3D: bounding disc per ordered triangle
+    bool has_runs = false;  // 3D: the pair records may name runs (host-built trees)
     const gq_cyl_t *run_cyl = nullptr;  // 3D: bounding cylinder of each run of a pair record, at the run's first triangle
     int32_t root_ref;
     float root_lo[3], root_hi[3];
@@ -88,9 +88,9 @@ cudaError_t launch_ray(const DevScene &s, int variant, const Tune &t, gq_vecs x,
 // Warp-coherent closest point; layout 0 = binary pairs, 1 / 2 = quantised 8-wide (3D): sorted / nearest first.
 cudaError_t launch_cp_packet(const DevScene &s, int layout, const Tune &t, gq_vecs q, int64_t n,
                              const int32_t *perm, const gq_cp_out &o, unsigned long long *counter, cudaStream_t st);
-// Fills tri_cyl[0 .. s.n_prims) and run_cyl[first of every run of the n_pairs pair records]
-// from the scene's device records (3D), on the default stream.
-cudaError_t build_cylinders(const DevScene &s, int64_t n_pairs, gq_cyl_t *tri_cyl, gq_cyl_t *run_cyl);
+// Fills run_cyl[first of every run of the n_pairs pair records] from the scene's device records
+// (3D), on the default stream.
+cudaError_t build_cylinders(const DevScene &s, int64_t n_pairs, gq_cyl_t *run_cyl);
 // Closest silhouette.  GQ_VARIANT_COHERENT (with a counter): warp-coherent traversal of
 // 32 sorted queries at a time; otherwise the reference order per lane, with persistent
 // lane refill when t.persist is set (t.budget steps between refills).
