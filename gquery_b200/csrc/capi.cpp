@@ -537,6 +537,7 @@ struct gq_batch {
 
     ~gq_batch() {
         DeviceGuard g(device);
+        gqi::FreeDuringCapture f;
         if (dev_scenes) cudaFree(dev_scenes);
         if (scratch) cudaFree(scratch);
         if (err) cudaFree(err);

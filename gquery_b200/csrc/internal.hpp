@@ -33,6 +33,15 @@ struct DeviceGuard {
     }
 };
 
+// While it lives, this thread may free device memory although some stream is being captured into
+// a graph: an object that goes meanwhile (a garbage collector's choice of moment) would
+// otherwise invalidate the capture.
+struct FreeDuringCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    FreeDuringCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~FreeDuringCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Stream-ordered memory of the query calls' scratch on one device.  The device's default pool
 // hands its memory back to the system at every synchronisation, and a call that follows
 // one maps it again: 16 points 675 us instead of 180 us, 8,388,608 rays 9 to 400 ms instead
@@ -88,6 +97,7 @@ struct gq_scene {
     ~gq_scene() {
         if (device < 0 || allocs.empty()) return;
         gqi::DeviceGuard g(device);
+        gqi::FreeDuringCapture f;
         if (pooled) gqi::scratch_pool_release(device);
         for (void *p : allocs) cudaFree(p);
     }

@@ -292,6 +292,7 @@ struct gq_server {
         if (worker.joinable()) worker.join();
         pool.stop();
         DeviceGuard g(device);
+        gqi::FreeDuringCapture f;
         for (Slot &s : slots) {
             if (s.st) cudaStreamSynchronize(s.st);
             if (s.done) cudaEventDestroy(s.done);
