@@ -687,15 +687,9 @@ cudaError_t launch_batch(const DevScene *scenes_dev, int n_scenes, BatchKind kin
         }
         // persistent warps in blocks of kBlock threads, whatever `block` is
         const size_t wsmem = (size_t)(kBlock / 32) * wsil::kWarpStack * sizeof(int2);
-        static int wbps = 0, w_sm = 0;
-        if (!wbps) {
-            int dev = 0, b = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&w_sm, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_batch_silw<D>, kBlock, wsmem);
-            wbps = b < 1 ? 1 : b;
-        }
-        const int64_t want = std::min<int64_t>((int64_t)wbps * w_sm, (kinds[2].n * 32 + kBlock - 1) / kBlock);
+        static std::atomic<int> known{0};
+        const int64_t blocks = resident_blocks(known, (const void *)k_batch_silw<D>, kBlock, wsmem);
+        const int64_t want = std::min<int64_t>(blocks, (kinds[2].n * 32 + kBlock - 1) / kBlock);
         k_batch_silw<D><<<dim3((unsigned)want), kBlock, wsmem, st>>>(scenes_dev, n_scenes, kinds[2], sil_out, counter,
                                                                      err);
         return cudaGetLastError();
@@ -711,15 +705,8 @@ cudaError_t launch_batch(const DevScene *scenes_dev, int n_scenes, BatchKind kin
                                     : (const void *)k_batch<D, RAYW, true, false>)
                              : (sil ? (const void *)k_batch<D, RAYW, false, true>
                                     : (const void *)k_batch<D, RAYW, false, false>);
-    static int bps_m[2][2][7] = {}, n_sm = 0;
-    if (!bps_m[bi][mi][si]) {
-        int dev = 0, b = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, block, smem);
-        bps_m[bi][mi][si] = b < 1 ? 1 : b;
-    }
-    const int bps = bps_m[bi][mi][si];
+    static std::atomic<int> known[2][2][7] = {};
+    const int64_t blocks = resident_blocks(known[bi][mi][si], kern, block, smem);
     const int64_t most = std::max(kinds[0].n, std::max(kinds[1].n, kinds[2].n));
     if (most <= 0) return cudaSuccess;
     // One warp per query as long as the GPU holds them (coherent tiles: one per 32 queries), where
@@ -731,9 +718,9 @@ cudaError_t launch_batch(const DevScene *scenes_dev, int n_scenes, BatchKind kin
         if (cp_mode != 1) warps = std::max(warps, kinds[0].n);
         warps = std::max(warps, kinds[1].n);
     }
-    int64_t want = std::min<int64_t>((int64_t)bps * n_sm, (warps * 32 + block - 1) / block);
+    int64_t want = std::min<int64_t>(blocks, (warps * 32 + block - 1) / block);
     if (grid_share > 0.f && grid_share < 1.f)
-        want = std::min<int64_t>(want, std::max<int64_t>(1, (int64_t)(grid_share * (float)(bps * n_sm))));
+        want = std::min<int64_t>(want, std::max<int64_t>(1, (int64_t)(grid_share * (float)blocks)));
     const int64_t have = std::max<int64_t>(1, want * (block / 32));
     auto lanes_of = [&](int64_t n) {
         return block == 32 ? 32 : (int)std::min<int64_t>(32, std::max<int64_t>(1, (n + have - 1) / have));
@@ -750,19 +737,13 @@ cudaError_t launch_batch(const DevScene *scenes_dev, int n_scenes, BatchKind kin
     if (e != cudaSuccess) return e;
     // the handed-over queries: persistent grids of one query per warp
     const size_t hsmem = (size_t)(block / 32) * wcp::kWarpStack * sizeof(int2);
-    static int hbps[2][2] = {};
-    if (!hbps[bi][0]) {
-        int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cp_heavy<D>, block, hsmem);
-        hbps[bi][0] = b < 1 ? 1 : b;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_sil_heavy<D>, block, hsmem);
-        hbps[bi][1] = b < 1 ? 1 : b;
-    }
+    static std::atomic<int> heavy[2][2] = {};
     auto hgrid = [&](int which, int64_t n) {
-        const int hb = hbps[bi][which];
-        int64_t g = std::min<int64_t>((int64_t)hb * n_sm, (n * 32 + block - 1) / block);
+        const int64_t room = resident_blocks(
+            heavy[bi][which], which ? (const void *)k_sil_heavy<D> : (const void *)k_cp_heavy<D>, block, hsmem);
+        int64_t g = std::min<int64_t>(room, (n * 32 + block - 1) / block);
         if (grid_share > 0.f && grid_share < 1.f)
-            g = std::min<int64_t>(g, std::max<int64_t>(1, (int64_t)(grid_share * (float)(hb * n_sm))));
+            g = std::min<int64_t>(g, std::max<int64_t>(1, (int64_t)(grid_share * (float)room)));
         return dim3((unsigned)g);
     };
     if (cp_mode == 2 && kinds[0].n > 0) {

@@ -63,20 +63,14 @@ __global__ void __maxnreg__(FORM == 2 ? 64 : 56) k_cp_packet(DevScene s, gq_vecs
 template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT = false, int FORM = 0>
 cudaError_t launch(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const int32_t *perm, const gq_cp_out &o,
                    unsigned long long *counter, cudaStream_t st) {
-    static int bps[3] = {0, 0, 0}, n_sm = 0;
     int block = t.block, slot = block_slot(block);
     if (slot < 0) slot = 1, block = 128;
     const size_t smem = FORM ? (size_t)(block / 32) * sizeof(pkt::LeafBuf) : 0;
-    if (!bps[slot]) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-        int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, FORM>, block, smem);
-        bps[slot] = b < 1 ? 1 : b;
-    }
+    static std::atomic<int> known[3] = {};
+    const int64_t blocks = resident_blocks(known[slot], (const void *)k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, FORM>,
+                                           block, smem);
     const int64_t warps = (n + 31) / 32;
-    const int64_t want = std::min<int64_t>((int64_t)bps[slot] * n_sm, (warps * 32 + block - 1) / block);
+    const int64_t want = std::min<int64_t>(blocks, (warps * 32 + block - 1) / block);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     k_cp_packet<D, LAYOUT, MINFIRST, STK, COMPACT, FORM><<<dim3((unsigned)want), block, smem, st>>>(s, q, n, perm, t.tiles, o,

@@ -731,7 +731,6 @@ cudaError_t morton_order(const DevScene &s, gq_vecs q, int64_t n, int32_t *perm,
 cudaError_t launch_sil(const DevScene &s, int variant, const Tune &t, gq_vecs x, const float *r_max, int64_t n,
                        const int32_t *perm, const gq_sil_out &o, unsigned long long *counter, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    static int bps[2][2][3] = {}, n_sm = 0;
     const int di = s.dim == 3 ? 1 : 0;
     int slot = block_slot(t.block), block = t.block;
     if (slot < 0) slot = 1, block = 128;
@@ -740,18 +739,14 @@ cudaError_t launch_sil(const DevScene &s, int variant, const Tune &t, gq_vecs x,
         using Fn = void (*)(DevScene, gq_vecs, const float *, int64_t, const int32_t *, gq_sil_out,
                             unsigned long long *);
         const Fn fn = s.dim == 3 ? k_sil_warp<3> : k_sil_warp<2>;
-        static int wb[2][3] = {}, w_sm = 0;
-        if (!wb[di][slot]) {
-            int dev = 0, b = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&w_sm, cudaDevAttrMultiProcessorCount, dev);
+        static std::atomic<int> known[2][3] = {};
+        if (known[di][slot].load(std::memory_order_relaxed) == 0) {
             // up to 8 warps x 4 KB of stacks (the opt-in keeps larger stacks possible)
             const int most = (kMaxBlock / 32) * wsil::kWarpStack * (int)sizeof(int2);
             cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void *)fn, block, smem);
-            wb[di][slot] = b < 1 ? 1 : b;
         }
-        const int64_t want = std::min<int64_t>((int64_t)wb[di][slot] * w_sm, (n * 32 + block - 1) / block);
+        const int64_t blocks = resident_blocks(known[di][slot], (const void *)fn, block, smem);
+        const int64_t want = std::min<int64_t>(blocks, (n * 32 + block - 1) / block);
         cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
         if (e != cudaSuccess) return e;
         fn<<<dim3((unsigned)want), block, smem, st>>>(s, x, r_max, n, perm, o, counter);
@@ -760,17 +755,11 @@ cudaError_t launch_sil(const DevScene &s, int variant, const Tune &t, gq_vecs x,
     const bool packet = variant == GQ_VARIANT_COHERENT && counter && n >= 32;
     const bool refill = !packet && t.persist && counter && n > 4096;
     if (packet || refill) {
-        const int ki = packet ? 1 : 0;
-        if (!bps[ki][di][slot]) {
-            int dev = 0, b = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-            const void *fn = packet ? (s.dim == 3 ? (const void *)k_sil_packet<3> : (const void *)k_sil_packet<2>)
-                                    : (s.dim == 3 ? (const void *)k_sil_persist<3> : (const void *)k_sil_persist<2>);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, block, 0);
-            bps[ki][di][slot] = b < 1 ? 1 : b;
-        }
-        const int64_t want = std::min<int64_t>((int64_t)bps[ki][di][slot] * n_sm, (n + block - 1) / block);
+        static std::atomic<int> known[2][2][3] = {};
+        const void *fn = packet ? (s.dim == 3 ? (const void *)k_sil_packet<3> : (const void *)k_sil_packet<2>)
+                                : (s.dim == 3 ? (const void *)k_sil_persist<3> : (const void *)k_sil_persist<2>);
+        const int64_t blocks = resident_blocks(known[packet ? 1 : 0][di][slot], fn, block, 0);
+        const int64_t want = std::min<int64_t>(blocks, (n + block - 1) / block);
         cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
         if (e != cudaSuccess) return e;
         const dim3 grid((unsigned)want);

@@ -1,6 +1,7 @@
 // Host-side launchers of the query kernels (implemented in queries.cu).
 #pragma once
 
+#include <atomic>
 #include <cuda_runtime.h>
 
 #include "../../../include/gq.h"
@@ -52,6 +53,22 @@ cudaError_t morton_order(const DevScene &s, gq_vecs q, int64_t n, int32_t *perm,
 // 13.4; 2D polylines gain nothing.  `ends` is an 8-byte device word.
 cudaError_t tile_order(const DevScene &s, gq_vecs q, int64_t n, const int32_t *perm, int32_t *tiles, int32_t *ends,
                        cudaStream_t st);
+
+// Blocks of `kernel` that the GPU holds at a time.  `known` is the launch form's static: 0 until
+// first asked, and set at once, since several host threads may launch a form for the first
+// time together (each finds the same number).
+inline int64_t resident_blocks(std::atomic<int> &known, const void *kernel, int block, size_t smem) {
+    int b = known.load(std::memory_order_relaxed);
+    if (b == 0) {
+        int dev = 0, n_sm = 0, per_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
+        b = (n_sm < 1 ? 1 : n_sm) * (per_sm < 1 ? 1 : per_sm);
+        known.store(b, std::memory_order_relaxed);
+    }
+    return b;
+}
 
 // Launch choices for one query kind (picked by the autotuner or the defaults).
 struct Tune {

@@ -229,15 +229,9 @@ __global__ void __launch_bounds__(kBlockG) k_ray_g8(DevScene s, gq_vecs a, gq_ve
 template <int D>
 cudaError_t launch(const DevScene &s, gq_vecs x, gq_vecs v, const float *r_max, int64_t n, const int32_t *perm,
                    const gq_ray_out &o, unsigned long long *counter, cudaStream_t st) {
-    static int bps = 0, n_sm = 0;
-    if (!bps) {
-        int dev = 0, b = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_ray_g8<D>, kBlockG, 0);
-        bps = b < 1 ? 1 : b;
-    }
-    const int64_t want = std::min<int64_t>((int64_t)bps * n_sm, (n * kG + kBlockG - 1) / kBlockG);
+    static std::atomic<int> known{0};
+    const int64_t blocks = resident_blocks(known, (const void *)k_ray_g8<D>, kBlockG, 0);
+    const int64_t want = std::min<int64_t>(blocks, (n * kG + kBlockG - 1) / kBlockG);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     k_ray_g8<D><<<dim3((unsigned)want), kBlockG, 0, st>>>(s, x, v, r_max, n, perm, o, counter);

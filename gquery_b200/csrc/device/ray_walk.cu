@@ -62,19 +62,12 @@ __global__ void __launch_bounds__(kBlockR, 6) k_ray_walk(DevScene s, gq_vecs a, 
 template <int D>
 cudaError_t launch(const DevScene &s, gq_vecs x, gq_vecs v, const float *r_max, int64_t n, const int32_t *perm,
                    const gq_ray_out &o, unsigned long long *counter, cudaStream_t st) {
-    static int bps = 0, n_sm = 0;
-    if (!bps) {
-        int dev = 0, b = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_ray_walk<D>, kBlockR, 0);
-        bps = b < 1 ? 1 : b;
-    }
-    const int64_t warps = (int64_t)bps * n_sm * (kBlockR / 32);
+    static std::atomic<int> known{0};
+    const int64_t blocks = resident_blocks(known, (const void *)k_ray_walk<D>, kBlockR, 0), warps = blocks * (kBlockR / 32);
     // fewer rays than lanes on the GPU: fewer per warp, so that they do not wait for one another
     const int lanes = (int)std::min<int64_t>(32, std::max<int64_t>(1, (n + warps - 1) / warps));
     const int refill = std::max(1, lanes / 4), leaves = std::max(1, lanes / 4);
-    const int64_t want = std::min<int64_t>((int64_t)bps * n_sm, ((n + lanes - 1) / lanes * 32 + kBlockR - 1) / kBlockR);
+    const int64_t want = std::min<int64_t>(blocks, ((n + lanes - 1) / lanes * 32 + kBlockR - 1) / kBlockR);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     k_ray_walk<D><<<dim3((unsigned)want), kBlockR, 0, st>>>(s, x, v, r_max, n, perm, o, counter, lanes, refill, leaves);

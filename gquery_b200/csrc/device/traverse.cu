@@ -94,15 +94,9 @@ cudaError_t launch_cfg(const DevScene &s, const Tune &t, gq_vecs a, gq_vecs b, c
     int slot = block_slot(t.block), block = t.block;
     if (slot < 0) slot = 1, block = 128;
     if (t.persist && counter && n > 4096) {
-        static int blocks_per_sm[3] = {0, 0, 0}, n_sm = 0;
-        if (!blocks_per_sm[slot]) {
-            int dev = 0, b = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trav_persist<D, RAY, WIDE, CFG>, block, 0);
-            blocks_per_sm[slot] = b < 1 ? 1 : b;
-        }
-        const int64_t want = std::min<int64_t>((int64_t)blocks_per_sm[slot] * n_sm, (n + block - 1) / block);
+        static std::atomic<int> known[3] = {};
+        const int64_t blocks = resident_blocks(known[slot], (const void *)k_trav_persist<D, RAY, WIDE, CFG>, block, 0);
+        const int64_t want = std::min<int64_t>(blocks, (n + block - 1) / block);
         cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
         if (e != cudaSuccess) return e;
         k_trav_persist<D, RAY, WIDE, CFG><<<dim3((unsigned)want), block, 0, st>>>(
