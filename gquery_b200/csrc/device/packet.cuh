@@ -125,15 +125,15 @@ __device__ __forceinline__ float cyl_bound(const float4 &c, const float4 &n, flo
 }
 
 // The bound a cylinder has to exceed for its triangles to be left untested: (sqrt(r) + eps)^2
-// for the squared radius r.  eps (2^-19 of the coordinates' size) is ten times the rounding
-// of cyl_bound and of the closest point that the triangle test forms together, so a triangle
-// that is left out would have had a key of at least r.  (The triangle test's barycentric
-// coordinates lose digits with the square of the distance over the triangle's size; up to a
-// thousand sizes away the point they give stays within the margin, and far beyond that its
-// own key means little.)
+// for the squared radius r, and the smallest normal number on top, below which the root is
+// taken of zero and squares lose their digits.  eps (2^-19 of the coordinates' size) is ten
+// times the rounding of cyl_bound and of the closest point that the triangle test forms
+// together, so a triangle that is left out would have had a key of at least r.  (The triangle
+// test's barycentric coordinates lose digits with the square of the distance over the
+// triangle's size, but the point they give stays in the triangle up to the margin.)
 __device__ __forceinline__ float cyl_limit(float r, float eps) {
     const float s = sqrt_approx(r) + eps;
-    return s * s;
+    return __fmaf_rn(s, s, 1.17549435e-38f);
 }
 
 // Squared distance from p to the closest point of triangle abc: the arithmetic of
