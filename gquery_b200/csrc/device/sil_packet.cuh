@@ -95,9 +95,9 @@ __device__ __forceinline__ void closest_silhouette(const DevScene &s, unsigned m
         }
         snch::PairView<D> P;
         snch::load_pair<D>(s, cur, P);
-        if (AHEAD) {
-            constexpr unsigned kPair = D == 3 ? sizeof(gq_spair3_t) : sizeof(gq_spair2_t);
-            constexpr unsigned kSil = D == 3 ? sizeof(gq_sile_t) : sizeof(gq_silv_t);
+        if constexpr (AHEAD) {
+            static_assert(D == 2, "measured for polylines only");
+            constexpr unsigned kPair = sizeof(gq_spair2_t), kSil = sizeof(gq_silv_t);
             const int cref = lane < 16 ? P.refs[0] : P.refs[1];
             const unsigned w = 16 * (lane & 15u);
             const char *from = (const char *)s.spairs + ((int64_t)(cref >= 0 ? cref : cur) * kPair + min(w, kPair - 4));
