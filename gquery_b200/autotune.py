@@ -57,12 +57,9 @@ def candidates(kind: str, dim: int, has_wide: bool, exact_stack: int, wide_stack
                 out.append(dict(variant="wide16", persist=1, budget=32, block=b))
         for b in blocks:
             out.append(dict(variant="exact", persist=1, budget=32, block=b))
-            if has_wide:
-                for budget in (16, 32, 64):
-                    out.append(dict(variant="wide8", persist=1, budget=budget, block=b))
-                out.append(dict(variant="wide8", persist=0, block=b))
         out.append(dict(variant="exact", persist=0, block=128))
         if has_wide:
+            out.append(dict(variant="wide8"))  # the default ray walk, whose launch has no choices
             out.append(dict(variant="wide8", packet=1))  # one ray per group of 8 lanes
             for packet in (0, 2):  # per lane; 2: while-while scheduling
                 out.append(dict(variant="wide8", packet=packet, sorted=0, persist=1, budget=32))  # nearest first
