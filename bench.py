@@ -10,7 +10,8 @@ kinds on two streams side by side; the same step kind after kind on one stream g
 per-kind breakdown, and the exact binary kernel (gQuery's visit order) and the quantised
 8-wide kernel are measured beside it that way.
 
-At one GPU the same line also carries (see --sections): c0 2D closest point on the
+The whole report goes to standard error as one JSON object; the line on standard output is its
+head and summary.  At one GPU the report also carries (see --sections): c0 2D closest point on the
 4,096-vertex star (every GPU variant and the CPU oracle), c2 closest silhouettes on the
 level-7 mesh (plain, refill, coherent), c3 512 uneven 2D scenes answered by one
 batched launch per step (eager and CUDA graph) against one plain call per scene and
@@ -663,6 +664,31 @@ def run_reference(args):
     return 0
 
 
+def headline(line):
+    """The line for standard output: the metric, what it was measured on, its end-to-end and
+    roofline figures and the summary, short enough (under 3,000 characters) for a reader that
+    keeps only the end of the output.  The whole report goes to standard error."""
+    def part(x, *keys):
+        return {k: x[k] for k in keys if k in x} if isinstance(x, dict) else x
+
+    def short(x):  # six digits where the figure is a comparison
+        if isinstance(x, dict):
+            return {k: short(v) for k, v in x.items()}
+        if isinstance(x, list):
+            return [short(v) for v in x]
+        return float(f"{x:.6g}") if isinstance(x, float) else x
+
+    out = part(line, "metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+               "scaling", "vs_baseline", "dtype", "data", "config", "clocks", "gpu_launches")
+    out["e2e"] = part(line.get("e2e"), "value", "unit", "ms_per_step", "h2d_bytes_per_step", "d2h_bytes_per_step",
+                      "lanes", "host_records_match")
+    out["roofline"] = short(part(line.get("roofline"), "bound", "achieved", "peak", "unit", "frac", "traffic", "kernel",
+                                 "peak_source"))
+    out["cpu_baseline"] = short(part(line.get("cpu_baseline"), "value", "unit", "cores", "kind"))
+    out["summary"] = short(line.get("summary"))
+    return out
+
+
 def summary(line):
     """The headline figures (variants against plain, error, serving tail), side by side,
     at the end of the line."""
@@ -1081,7 +1107,8 @@ def main():
                 line[key] = fn()
                 line[key]["section_wall_s"] = time.perf_counter() - t_sec
         line["summary"] = summary(line)
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
