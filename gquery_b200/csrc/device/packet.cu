@@ -95,9 +95,10 @@ constexpr int64_t kAheadBelow2D = 1 << 21, kSmallCall2D = 1 << 16, kLargeLine = 
 template <int D, int LAYOUT, bool MINFIRST>
 cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const int32_t *perm,
                        const gq_cp_out &o, unsigned long long *counter, cudaStream_t st) {
+    constexpr int kForm = D == 3 ? 1 : 0;  // triangles as pairs
     if (t.packet == 2) {  // the compact stack (FP16 keys, one node word per warp)
-        if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32, true>(s, t, q, n, perm, o, counter, st);
-        return launch<D, LAYOUT, MINFIRST, pkt::kPStack, true>(s, t, q, n, perm, o, counter, st);
+        if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32, true, kForm>(s, t, q, n, perm, o, counter, st);
+        return launch<D, LAYOUT, MINFIRST, pkt::kPStack, true, kForm>(s, t, q, n, perm, o, counter, st);
     }
     if constexpr (LAYOUT == 0) {
         const bool ahead = D == 3 ? n < (s.has_runs ? kAheadBelow3D : kAheadNoRuns)
@@ -105,12 +106,9 @@ cudaError_t launch_stk(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, c
         if (ahead)
             return t.stack == 32 ? launch<D, LAYOUT, MINFIRST, 32, false, 2>(s, t, q, n, perm, o, counter, st)
                                  : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, 2>(s, t, q, n, perm, o, counter, st);
-        if constexpr (D == 3)
-            return t.stack == 32 ? launch<D, LAYOUT, MINFIRST, 32, false, 1>(s, t, q, n, perm, o, counter, st)
-                                 : launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, 1>(s, t, q, n, perm, o, counter, st);
     }
-    if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32>(s, t, q, n, perm, o, counter, st);
-    return launch<D, LAYOUT, MINFIRST, pkt::kPStack>(s, t, q, n, perm, o, counter, st);
+    if (t.stack == 32) return launch<D, LAYOUT, MINFIRST, 32, false, kForm>(s, t, q, n, perm, o, counter, st);
+    return launch<D, LAYOUT, MINFIRST, pkt::kPStack, false, kForm>(s, t, q, n, perm, o, counter, st);
 }
 
 // Bounding cylinder of triangles [first, first + count) (gq_cyl_t), in double, rounded
