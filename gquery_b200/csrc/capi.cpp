@@ -775,7 +775,10 @@ gq_status gq_closest_point(const gq_scene *s, gq_vecs q, int64_t n, const gq_cp_
     // up to one tile of the coherent walk: its answers do not depend on the order within
     const bool any_order = v == GQ_VARIANT_COHERENT && n <= 32;
     gqd::Tune tune = to_tune(s, GQ_KIND_CLOSEST_POINT, v);
-    const bool middle_first = v == GQ_VARIANT_COHERENT && s->dim == 3;  // 19.0 -> 18.2 ms for 8,388,608 points
+    // 8,388,608 points on 1,310,720 and 327,680 triangles 19.0 -> 17.5 and 11.6 -> 10.1 ms, 4,194,304 13.1 -> 11.8
+    // and 7.9 -> 6.8 (near the surface within 4% either way); 2,097,157 10.3 -> 9.6 and 5.7 -> 4.8, but 1,048,576
+    // 9.5 -> 10.1, and near 161,920 triangles, half of them slivers, 1.82 -> 1.97
+    const bool middle_first = v == GQ_VARIANT_COHERENT && s->dim == 3;
     if ((st = prepare_order(s, q, n, opts, cs, scr, &perm, &counter, nullptr, any_order,
                             middle_first && n >= (1 << 22) ? &tune.tiles : nullptr)) != GQ_OK)
         return st;

@@ -179,8 +179,15 @@ __device__ __noinline__ void sil_warp_phase(const DevScene *scenes, int n_scenes
 // Closest-point queries whose per-lane traversal passes this many node visits are
 // handed to k_cp_heavy (cp_mode 2).
 constexpr int kHeavyVisits = 1024;
-// Queries of one kind from which they are sorted where the order does not change their
-// answers, and rays of 2D scenes on the default walk (traverse.cu, ray_any_order).
+// Queries of one kind from which they are sorted where the order does not change their answers.
+// Never / always sorted, ms, 8 meshes and 16 polylines of 65,536 segments: closest points 32,768
+// 0.52 / 0.66 and 0.86 / 1.07, 131,072 0.84 / 1.05 and 1.13 / 1.63; one silhouette per warp 32,768 0.65 / 0.82 and
+// 0.44 / 0.55, 65,536 1.24 / 1.22 and 0.77 / 0.75, 262,144 4.08 / 3.89 and 2.11 / 2.00; all kinds together 65,536 1.58 /
+// 1.67 and 1.49 / 2.05, 131,072 2.57 / 2.50 and 2.21 / 2.64, 262,144 4.79 / 4.55 and 3.84 / 3.46.
+// So a step alone would be sorted from 131,072 on; beside other steps the sorted walks leave those
+// more of the GPU (the server, whose large requests start at 32,768: saturation 114.0 Mq/s with the
+// line at 32,768, 111.8 at 131,072, means of three runs; half the requests at 80% within 1.97 / 2.04 ms).
+// Rays of 2D scenes on the default walk: traverse.cu, ray_any_order.
 constexpr int64_t kSortFrom = 1 << 15, kSortFrom2D = 1 << 18;
 // Node visits (closest points, rays) or steps (silhouettes) between refills in k_batch.
 constexpr int kBudget = 32;
