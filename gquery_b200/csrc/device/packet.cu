@@ -86,9 +86,9 @@ cudaError_t launch(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const
 // Device-built trees, one triangle per leaf, leave it out earlier: 327,680 curved and 200,000
 // scattered triangles, 262,144 points 7.3 / 6.7 and 0.55 / 0.55 ms, 1,048,576 8.4 / 8.0 and 0.69 / 0.80.
 // All forms give the same answers bit for bit.
-// 2D (no pairs): 100,003 points on 60,000 segments 842 / 581 us without / with, 2,000,003 on 262,144
-// 3.24 / 2.86 ms, but 1,048,576 on 4,096, whose tree stays in L1 anyway, 249 / 260 us, so
-// polylines below 16,384 segments leave it out from 65,536 points on, the others from 2,097,152.
+// 2D (no pairs), without / with, us: 65,536 points on 4,096 / 16,384 / 65,536 segments 164 / 144, 311 / 236 and
+// 905 / 624, 1,048,576 points 260 / 271, 404 / 393 and 856 / 768 (8,192 segments 305 / 313: a tree that stays in
+// L1 anyway), 4,194,304 on 65,536 1,890 / 1,913.
 constexpr int64_t kAheadBelow3D = 1 << 22, kAheadNoRuns = 1 << 19;
 constexpr int64_t kAheadBelow2D = 1 << 21, kSmallCall2D = 1 << 16, kLargeLine = 1 << 14;
 
