@@ -7,7 +7,6 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
-#include <map>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -41,10 +40,12 @@ struct ScratchPool {
     int scenes = 0;
 };
 std::mutex g_pool_mu;
-std::map<int, ScratchPool> g_pools;  // by device
+constexpr int kPoolDevices = 64;
+ScratchPool g_pools[kPoolDevices];  // a scene on a device beyond has the device's default pool
 }  // namespace
 
 cudaMemPool_t scratch_pool_retain(int device) {
+    if (device < 0 || device >= kPoolDevices) return nullptr;
     std::lock_guard<std::mutex> lk(g_pool_mu);
     ScratchPool &e = g_pools[device];
     if (e.scenes++ == 0) {
@@ -64,11 +65,12 @@ cudaMemPool_t scratch_pool_retain(int device) {
 }
 
 void scratch_pool_release(int device) {
+    if (device < 0 || device >= kPoolDevices) return;
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    auto it = g_pools.find(device);
-    if (it == g_pools.end() || --it->second.scenes > 0) return;
-    if (it->second.pool) cudaMemPoolDestroy(it->second.pool);  // pending frees finish first
-    g_pools.erase(it);
+    ScratchPool &e = g_pools[device];
+    if (--e.scenes > 0) return;
+    if (e.pool) cudaMemPoolDestroy(e.pool);  // pending frees finish first
+    e.pool = nullptr;
 }
 }  // namespace gqi
 
