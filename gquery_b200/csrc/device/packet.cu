@@ -177,6 +177,11 @@ __device__ void cylinder_of(const gq_tri_t *prims, int64_t first, int count, gq_
     out.half = ok ? __double2float_ru(half + slack) : kInf;
 }
 
+__global__ void __launch_bounds__(128) k_no_cyl(gq_cyl_t *out, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = gq_cyl_t{0.f, 0.f, 0.f, kInf, 0.f, 0.f, 0.f, kInf};
+}
+
 // The walk meets the largest runs only: the two runs of a pair that is itself inside a run
 // are left out (they may start at the same triangle as the run around them).
 __global__ void __launch_bounds__(128) k_run_cyl(const gq_pair3_t *pairs, int64_t n, int32_t root, const gq_tri_t *prims,
@@ -194,6 +199,10 @@ __global__ void __launch_bounds__(128) k_run_cyl(const gq_pair3_t *pairs, int64_
 }  // namespace
 
 cudaError_t build_cylinders(const DevScene &s, int64_t n_pairs, gq_cyl_t *run_cyl) {
+    // whatever runs the records of a file name, a place without a cylinder bounds nothing
+    k_no_cyl<<<dim3((unsigned)((s.n_prims + 127) / 128)), 128>>>(run_cyl, s.n_prims);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
     if (n_pairs > 0)
         k_run_cyl<<<dim3((unsigned)((2 * n_pairs + 127) / 128)), 128>>>(
             static_cast<const gq_pair3_t *>(s.pairs), n_pairs, s.root_ref, static_cast<const gq_tri_t *>(s.prims),
