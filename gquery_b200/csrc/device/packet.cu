@@ -15,10 +15,11 @@ __device__ __forceinline__ float qget(const gq_vecs &v, int64_t i, int k) {
     return v.ptr[(int64_t)k * v.comp_stride + i * v.elem_stride];
 }
 
-// Registers: 56 keep 36 warps on an SM; the form that fetches ahead needs 64 for its loops and is
-// bound by latency.
+// Registers: 56 keep 36 warps on an SM; the form that fetches ahead is bound by latency and takes 65
+// (at most 64 / 72: 2,003 points on 327,680 triangles 2.13 / 2.10 ms, 1,048,576 on 20,480 0.94 / 0.90,
+// 1,048,576 on 161,920 2.75 / 2.65).
 template <int D, int LAYOUT, bool MINFIRST, int STK, bool COMPACT, int FORM>
-__global__ void __maxnreg__(FORM == 2 ? 64 : 56) k_cp_packet(DevScene s, gq_vecs q, int64_t n, const int32_t *perm, const int32_t *tiles,
+__global__ void __maxnreg__(FORM == 2 ? 72 : 56) k_cp_packet(DevScene s, gq_vecs q, int64_t n, const int32_t *perm, const int32_t *tiles,
                                                          gq_cp_out o, unsigned long long *counter) {
     const unsigned lane = threadIdx.x & 31u;
     // (ref, this lane's key) per entry; refs are the same in every lane
@@ -79,17 +80,18 @@ cudaError_t launch(const DevScene &s, const Tune &t, gq_vecs q, int64_t n, const
 }
 
 // Calls of fewer queries bring children into L1 ahead (packet.cuh): their time is the latency of
-// the heaviest tiles; from here on the GPU has some thirty tiles per resident warp and the
-// form with more warps wins.  Without / with, uniform points on 1,310,720 triangles and on a tube
-// of 320,000 slivers: 2,097,157 10.0 / 8.8 and 22.0 / 21.2 ms, 4,194,304 12.4 / 12.1 and 24.6 / 26.5,
-// 6,000,000 14.4 / 14.8 and 30.5 / 32.6, 8,388,608 17.5 / 19.5 and 39.4 / 41.7.
+// the heaviest tiles; from here on the GPU has some fifteen tiles per resident warp and the
+// form with more warps wins where it matters.  Without / with, uniform points on 1,310,720 curved
+// and 200,000 scattered triangles and on a tube of 320,000 slivers: 1,048,576 8.6 / 7.6, 0.69 / 0.68 and 16.6 / 15.7
+// ms, 2,097,157 9.8 / 10.2, 1.05 / 1.09 and 21.6 / 20.1, 3,000,000 11.2 / 13.3, 1.49 / 1.52 and 25.0 / 23.9,
+// 4,000,000 12.3 / 14.3, 2.05 / 2.08 and 29.6 / 28.1.
 // Device-built trees, one triangle per leaf, leave it out earlier: 327,680 curved and 200,000
 // scattered triangles, 262,144 points 7.3 / 6.7 and 0.55 / 0.55 ms, 1,048,576 8.4 / 8.0 and 0.69 / 0.80.
 // All forms give the same answers bit for bit.
 // 2D (no pairs), without / with, us: 65,536 points on 4,096 / 16,384 / 65,536 segments 164 / 144, 311 / 236 and
 // 905 / 624, 1,048,576 points 260 / 271, 404 / 393 and 856 / 768 (8,192 segments 305 / 313: a tree that stays in
 // L1 anyway), 4,194,304 on 65,536 1,890 / 1,913.
-constexpr int64_t kAheadBelow3D = 1 << 22, kAheadNoRuns = 1 << 19;
+constexpr int64_t kAheadBelow3D = 1 << 21, kAheadNoRuns = 1 << 19;
 constexpr int64_t kAheadBelow2D = 1 << 21, kSmallCall2D = 1 << 16, kLargeLine = 1 << 14;
 
 template <int D, int LAYOUT, bool MINFIRST>
